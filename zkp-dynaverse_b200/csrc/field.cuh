@@ -2,11 +2,25 @@
 //
 // Multiplication is CIOS (Koc, Acar, Kaliski, "Analyzing and comparing
 // Montgomery multiplication algorithms", 1996) written as PTX carry chains.
-// Each row "t += x * v" is split into an even-limb chain (lo of v0,v2,.. into
-// t0,t2,..; hi into t1,t3,..) and an odd-limb chain, so every chain is a
-// single uninterrupted mad.lo.cc / madc.hi.cc sequence.  p < 2^254, so the
-// 9-limb accumulator never overflows (T < 2p before each row, and
-// T + a*b_i + m*p < 2^288).
+// What bounds it is the 32x32 -> 64-bit multiply-add: four cycles a warp on
+// each SM quarter with a carry or without, 6.2 for a lone warp; FP64
+// products on 24-bit or 52-bit limbs come out no faster on this part, and
+// share issue slots with the integer ones.  So the layout removes what is
+// not a product:
+//  - The running sum is two accumulators, T = E + 2^32 O, that take the
+//    products with the even and with the odd limbs of a row.  A 64-bit product
+//    then always lands on an even-aligned register pair (one multiply-add
+//    instruction), also after the shift by one limb, which makes O the new
+//    E and E without two limbs the new O: no moves, no re-split additions.
+//  - With N = (p (-p^-1 mod 2^32) + 1) / 2^32, T + t0 p (-p^-1 mod 2^32) is
+//    divisible by 2^32 and its quotient is (T >> 32) + t0 N (t0 the low limb):
+//    a reduction step needs no product for its multiplier.  N < p, but the
+//    steps no longer keep T below 2p, so the last two take the multiplier
+//    m = -t0 / p mod 2^32 and p.  Bounds: T < 2^33 p < 2^288 before every
+//    step, below 2p after the last.
+// Measured (148 x 512 threads, pairs of products): 53.3 to 64.4 G products/s,
+// against 68.8 that the multiply-adds alone would allow; one warp alone,
+// 505 to 449 ns a product (single accumulator to this form).
 //
 // Values are kept fully reduced in [0, p).
 #pragma once
@@ -32,6 +46,16 @@ struct FrCfg {
 };
 
 #define DV_INL __device__ __forceinline__
+
+// Operands of a 16-word asm statement r <- a op b.
+#define DV_WIDE_OPERANDS(r, a, b)                                                                                     \
+    : "=&r"(r.v[0]), "=&r"(r.v[1]), "=&r"(r.v[2]), "=&r"(r.v[3]), "=&r"(r.v[4]), "=&r"(r.v[5]), "=&r"(r.v[6]),       \
+      "=&r"(r.v[7]), "=&r"(r.v[8]), "=&r"(r.v[9]), "=&r"(r.v[10]), "=&r"(r.v[11]), "=&r"(r.v[12]), "=&r"(r.v[13]),   \
+      "=&r"(r.v[14]), "=&r"(r.v[15])                                                                                  \
+    : "r"(a.v[0]), "r"(a.v[1]), "r"(a.v[2]), "r"(a.v[3]), "r"(a.v[4]), "r"(a.v[5]), "r"(a.v[6]), "r"(a.v[7]),        \
+      "r"(a.v[8]), "r"(a.v[9]), "r"(a.v[10]), "r"(a.v[11]), "r"(a.v[12]), "r"(a.v[13]), "r"(a.v[14]), "r"(a.v[15]),  \
+      "r"(b.v[0]), "r"(b.v[1]), "r"(b.v[2]), "r"(b.v[3]), "r"(b.v[4]), "r"(b.v[5]), "r"(b.v[6]), "r"(b.v[7]),        \
+      "r"(b.v[8]), "r"(b.v[9]), "r"(b.v[10]), "r"(b.v[11]), "r"(b.v[12]), "r"(b.v[13]), "r"(b.v[14]), "r"(b.v[15])
 
 // Two results of a paired multiplication.
 template <class T>
@@ -154,60 +178,28 @@ struct __align__(16) Fp {  // 16-byte aligned: global copies move as 128-bit acc
         return a.is_zero() ? a : sub(z, a);
     }
 
+    // T = a b_0, then eight steps of reduction, the first seven each followed by T += a b_(i+1).
     DV_INL static Fp mul_inl(const Fp& a, const Fp& b) {
-        uint32_t t0 = 0, t1 = 0, t2 = 0, t3 = 0, t4 = 0, t5 = 0, t6 = 0, t7 = 0, t8 = 0;
+        constexpr Words N = reduction_words();
+        uint32_t e[8], o[8], t[8];
+        mul4(e, a.v[0], a.v[2], a.v[4], a.v[6], b.v[0]);
+        mul4(o, a.v[1], a.v[3], a.v[5], a.v[7], b.v[0]);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const uint32_t bi = b.v[i];
-            asm("mad.lo.cc.u32 %0, %9, %13, %0;\n\t"
-                "madc.hi.cc.u32 %1, %9, %13, %1;\n\t"
-                "madc.lo.cc.u32 %2, %10, %13, %2;\n\t"
-                "madc.hi.cc.u32 %3, %10, %13, %3;\n\t"
-                "madc.lo.cc.u32 %4, %11, %13, %4;\n\t"
-                "madc.hi.cc.u32 %5, %11, %13, %5;\n\t"
-                "madc.lo.cc.u32 %6, %12, %13, %6;\n\t"
-                "madc.hi.cc.u32 %7, %12, %13, %7;\n\t"
-                "addc.u32 %8, %8, 0;"
-                : "+r"(t0), "+r"(t1), "+r"(t2), "+r"(t3), "+r"(t4), "+r"(t5), "+r"(t6), "+r"(t7), "+r"(t8)
-                : "r"(a.v[0]), "r"(a.v[2]), "r"(a.v[4]), "r"(a.v[6]), "r"(bi));
-            asm("mad.lo.cc.u32 %0, %8, %12, %0;\n\t"
-                "madc.hi.cc.u32 %1, %8, %12, %1;\n\t"
-                "madc.lo.cc.u32 %2, %9, %12, %2;\n\t"
-                "madc.hi.cc.u32 %3, %9, %12, %3;\n\t"
-                "madc.lo.cc.u32 %4, %10, %12, %4;\n\t"
-                "madc.hi.cc.u32 %5, %10, %12, %5;\n\t"
-                "madc.lo.cc.u32 %6, %11, %12, %6;\n\t"
-                "madc.hi.u32 %7, %11, %12, %7;"
-                : "+r"(t1), "+r"(t2), "+r"(t3), "+r"(t4), "+r"(t5), "+r"(t6), "+r"(t7), "+r"(t8)
-                : "r"(a.v[1]), "r"(a.v[3]), "r"(a.v[5]), "r"(a.v[7]), "r"(bi));
-            const uint32_t m = t0 * C::INV;
-            asm("mad.lo.cc.u32 %0, %9, %10, %0;\n\t"
-                "madc.hi.cc.u32 %1, %9, %10, %1;\n\t"
-                "madc.lo.cc.u32 %2, %9, %11, %2;\n\t"
-                "madc.hi.cc.u32 %3, %9, %11, %3;\n\t"
-                "madc.lo.cc.u32 %4, %9, %12, %4;\n\t"
-                "madc.hi.cc.u32 %5, %9, %12, %5;\n\t"
-                "madc.lo.cc.u32 %6, %9, %13, %6;\n\t"
-                "madc.hi.cc.u32 %7, %9, %13, %7;\n\t"
-                "addc.u32 %8, %8, 0;"
-                : "+r"(t0), "+r"(t1), "+r"(t2), "+r"(t3), "+r"(t4), "+r"(t5), "+r"(t6), "+r"(t7), "+r"(t8)
-                : "r"(m), "n"(C::P0), "n"(C::P2), "n"(C::P4), "n"(C::P6));
-            asm("mad.lo.cc.u32 %0, %8, %9, %0;\n\t"
-                "madc.hi.cc.u32 %1, %8, %9, %1;\n\t"
-                "madc.lo.cc.u32 %2, %8, %10, %2;\n\t"
-                "madc.hi.cc.u32 %3, %8, %10, %3;\n\t"
-                "madc.lo.cc.u32 %4, %8, %11, %4;\n\t"
-                "madc.hi.cc.u32 %5, %8, %11, %5;\n\t"
-                "madc.lo.cc.u32 %6, %8, %12, %6;\n\t"
-                "madc.hi.u32 %7, %8, %12, %7;"
-                : "+r"(t1), "+r"(t2), "+r"(t3), "+r"(t4), "+r"(t5), "+r"(t6), "+r"(t7), "+r"(t8)
-                : "r"(m), "n"(C::P1), "n"(C::P3), "n"(C::P5), "n"(C::P7));
-            // t0 is now 0 (mod 2^32): shift one limb down.
-            t0 = t1; t1 = t2; t2 = t3; t3 = t4; t4 = t5; t5 = t6; t6 = t7; t7 = t8; t8 = 0;
+        for (int i = 0; i < 6; ++i) {
+            const uint32_t t0 = e[0];
+            shift_mac4(t, o, e, N.v[1], N.v[3], N.v[5], N.v[7], t0);
+            mac4_top(o, t[7], N.v[0], N.v[2], N.v[4], N.v[6], t0);
+            mac4(t, a.v[1], a.v[3], a.v[5], a.v[7], b.v[i + 1]);
+            mac4_top(o, t[7], a.v[0], a.v[2], a.v[4], a.v[6], b.v[i + 1]);
+            rotate(e, o, t);
         }
+        reduce_step(e, o);
+        shift_mac4(t, o, e, a.v[1], a.v[3], a.v[5], a.v[7], b.v[7]);
+        mac4_top(o, t[7], a.v[0], a.v[2], a.v[4], a.v[6], b.v[7]);
+        rotate(e, o, t);
+        reduce_step(e, o);
         Fp r;
-        r.v[0] = t0; r.v[1] = t1; r.v[2] = t2; r.v[3] = t3;
-        r.v[4] = t4; r.v[5] = t5; r.v[6] = t6; r.v[7] = t7;
+        merge(r.v, e, o);
         reduce_once(r.v);
         return r;
     }
@@ -231,90 +223,145 @@ struct __align__(16) Fp {  // 16-byte aligned: global copies move as 128-bit acc
         return {mul_inl(a, b), mul_inl(c, d)};
     }
 #endif
-    // Montgomery square: the cross products a_i a_j (i < j) once, summed by
-    // columns in a three-word accumulator, doubled by a one-bit shift, plus
-    // the diagonal a_i^2 in one carry chain; then eight word-by-word
-    // reduction steps over the 512-bit square (two interleaved carry chains
-    // per step as in mul_inl, e carrying into the word above the window).
-    // 36 + 72 word products against a product's 136.
-    DV_INL static Fp sqr_inl(const Fp& a) {
-        uint32_t t[16];
-        uint32_t c0 = 0, c1 = 0, c2 = 0;
-        t[0] = 0;
+    // 512-bit values: products that are added or subtracted before one
+    // reduction (redc) instead of one each.
+    struct Wide {
+        uint32_t v[16];
+    };
+    DV_INL static Wide mul_wide(const Fp& a, const Fp& b) {
+        const uint32_t ae[4] = {a.v[0], a.v[2], a.v[4], a.v[6]}, ao[4] = {a.v[1], a.v[3], a.v[5], a.v[7]};
+        uint32_t e[17], o[17];  // word 16 only ever takes zero carries
 #pragma unroll
-        for (int k = 1; k < 14; ++k) {
+        for (int j = 8; j < 17; ++j) e[j] = o[j] = 0;
+        mul4(e, ae[0], ae[1], ae[2], ae[3], b.v[0]);
+        mul4(o, ao[0], ao[1], ao[2], ao[3], b.v[0]);
 #pragma unroll
-            for (int i = (k > 7 ? k - 7 : 0); 2 * i < k; ++i)
-                asm("mad.lo.cc.u32 %0, %3, %4, %0;\n\t"
-                    "madc.hi.cc.u32 %1, %3, %4, %1;\n\t"
-                    "addc.u32 %2, %2, 0;"
-                    : "+r"(c0), "+r"(c1), "+r"(c2)
-                    : "r"(a.v[i]), "r"(a.v[k - i]));
-            t[k] = c0;
-            c0 = c1;
-            c1 = c2;
-            c2 = 0;
+        for (int i = 1; i < 8; ++i) {
+            if (i & 1) {  // even limbs of a at odd positions, odd limbs at even ones
+                chain<4>(o + i - 1, ae, b.v[i], o[i + 7]);
+                chain<4>(e + i + 1, ao, b.v[i], e[i + 9 < 16 ? i + 9 : 16]);
+            } else {
+                chain<4>(e + i, ae, b.v[i], e[i + 8]);
+                chain<4>(o + i, ao, b.v[i], o[i + 8]);
+            }
         }
-        t[14] = c0;
-        t[15] = c1;
+        return combine(e, o);
+    }
+    // a^2 as rows a_i (a_i, then the doubled limbs above i): 36 products.
+    DV_INL static Wide sqr_wide(const Fp& a) {
+        uint32_t e[17], o[17], d[8], s[8];  // d: limbs of 2a; s: a_j << 1, without the bit from below
 #pragma unroll
-        for (int k = 15; k > 0; --k) t[k] = __funnelshift_l(t[k - 1], t[k], 1);
-        asm("mad.lo.cc.u32 %0, %16, %16, %0;\n\t"
-            "madc.hi.cc.u32 %1, %16, %16, %1;\n\t"
-            "madc.lo.cc.u32 %2, %17, %17, %2;\n\t"
-            "madc.hi.cc.u32 %3, %17, %17, %3;\n\t"
-            "madc.lo.cc.u32 %4, %18, %18, %4;\n\t"
-            "madc.hi.cc.u32 %5, %18, %18, %5;\n\t"
-            "madc.lo.cc.u32 %6, %19, %19, %6;\n\t"
-            "madc.hi.cc.u32 %7, %19, %19, %7;\n\t"
-            "madc.lo.cc.u32 %8, %20, %20, %8;\n\t"
-            "madc.hi.cc.u32 %9, %20, %20, %9;\n\t"
-            "madc.lo.cc.u32 %10, %21, %21, %10;\n\t"
-            "madc.hi.cc.u32 %11, %21, %21, %11;\n\t"
-            "madc.lo.cc.u32 %12, %22, %22, %12;\n\t"
-            "madc.hi.cc.u32 %13, %22, %22, %13;\n\t"
-            "madc.lo.cc.u32 %14, %23, %23, %14;\n\t"
-            "madc.hi.u32 %15, %23, %23, %15;"
-            : "+r"(t[0]), "+r"(t[1]), "+r"(t[2]), "+r"(t[3]), "+r"(t[4]), "+r"(t[5]), "+r"(t[6]), "+r"(t[7]),
-              "+r"(t[8]), "+r"(t[9]), "+r"(t[10]), "+r"(t[11]), "+r"(t[12]), "+r"(t[13]), "+r"(t[14]), "+r"(t[15])
-            : "r"(a.v[0]), "r"(a.v[1]), "r"(a.v[2]), "r"(a.v[3]), "r"(a.v[4]), "r"(a.v[5]), "r"(a.v[6]),
-              "r"(a.v[7]));
-        uint32_t e = 0;  // carry into t[i + 8] at step i
+        for (int j = 1; j < 8; ++j) {
+            d[j] = __funnelshift_l(a.v[j - 1], a.v[j], 1);
+            s[j] = a.v[j] << 1;
+        }
+#pragma unroll
+        for (int j = 0; j < 17; ++j) e[j] = o[j] = 0;
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
-            const uint32_t m = t[i] * C::INV;
-            asm("mad.lo.cc.u32 %0, %10, %11, %0;\n\t"
-                "madc.hi.cc.u32 %1, %10, %11, %1;\n\t"
-                "madc.lo.cc.u32 %2, %10, %12, %2;\n\t"
-                "madc.hi.cc.u32 %3, %10, %12, %3;\n\t"
-                "madc.lo.cc.u32 %4, %10, %13, %4;\n\t"
-                "madc.hi.cc.u32 %5, %10, %13, %5;\n\t"
-                "madc.lo.cc.u32 %6, %10, %14, %6;\n\t"
-                "madc.hi.cc.u32 %7, %10, %14, %7;\n\t"
-                "addc.cc.u32 %8, %8, %9;\n\t"
-                "addc.u32 %9, 0, 0;"
-                : "+r"(t[i]), "+r"(t[i + 1]), "+r"(t[i + 2]), "+r"(t[i + 3]), "+r"(t[i + 4]), "+r"(t[i + 5]),
-                  "+r"(t[i + 6]), "+r"(t[i + 7]), "+r"(t[i + 8]), "+r"(e)
-                : "r"(m), "n"(C::P0), "n"(C::P2), "n"(C::P4), "n"(C::P6));
-            asm("mad.lo.cc.u32 %0, %9, %10, %0;\n\t"
-                "madc.hi.cc.u32 %1, %9, %10, %1;\n\t"
-                "madc.lo.cc.u32 %2, %9, %11, %2;\n\t"
-                "madc.hi.cc.u32 %3, %9, %11, %3;\n\t"
-                "madc.lo.cc.u32 %4, %9, %12, %4;\n\t"
-                "madc.hi.cc.u32 %5, %9, %12, %5;\n\t"
-                "madc.lo.cc.u32 %6, %9, %13, %6;\n\t"
-                "madc.hi.cc.u32 %7, %9, %13, %7;\n\t"
-                "addc.u32 %8, %8, 0;"
-                : "+r"(t[i + 1]), "+r"(t[i + 2]), "+r"(t[i + 3]), "+r"(t[i + 4]), "+r"(t[i + 5]), "+r"(t[i + 6]),
-                  "+r"(t[i + 7]), "+r"(t[i + 8]), "+r"(e)
-                : "r"(m), "n"(C::P1), "n"(C::P3), "n"(C::P5), "n"(C::P7));
-        }
-        Fp r;
+            uint32_t x[4] = {a.v[i], 0, 0, 0}, y[4] = {0, 0, 0, 0};
+            int nx = 1, ny = 0;
+            if (i < 7) y[ny++] = s[i + 1];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) r.v[j] = t[8 + j];
+            for (int j = i + 2; j < 8; j += 2) x[nx++] = d[j];
+#pragma unroll
+            for (int j = i + 3; j < 8; j += 2) y[ny++] = d[j];
+            if (nx == 4) chain<4>(e + 2 * i, x, a.v[i], e[2 * i + 8]);
+            else if (nx == 3) chain<3>(e + 2 * i, x, a.v[i], e[2 * i + 6]);
+            else if (nx == 2) chain<2>(e + 2 * i, x, a.v[i], e[2 * i + 4]);
+            else chain<1>(e + 2 * i, x, a.v[i], e[2 * i + 2]);
+            if (ny == 4) chain<4>(o + 2 * i, y, a.v[i], o[2 * i + 8]);
+            else if (ny == 3) chain<3>(o + 2 * i, y, a.v[i], o[2 * i + 6]);
+            else if (ny == 2) chain<2>(o + 2 * i, y, a.v[i], o[2 * i + 4]);
+            else if (ny == 1) chain<1>(o + 2 * i, y, a.v[i], o[2 * i + 2]);
+        }
+        return combine(e, o);
+    }
+    // a + b and a - b modulo 2^512 (two's complement)
+    DV_INL static Wide wide_add(const Wide& a, const Wide& b) {
+        Wide r;
+        asm("add.cc.u32 %0, %16, %32;\n\taddc.cc.u32 %1, %17, %33;\n\taddc.cc.u32 %2, %18, %34;\n\t"
+            "addc.cc.u32 %3, %19, %35;\n\taddc.cc.u32 %4, %20, %36;\n\taddc.cc.u32 %5, %21, %37;\n\t"
+            "addc.cc.u32 %6, %22, %38;\n\taddc.cc.u32 %7, %23, %39;\n\taddc.cc.u32 %8, %24, %40;\n\t"
+            "addc.cc.u32 %9, %25, %41;\n\taddc.cc.u32 %10, %26, %42;\n\taddc.cc.u32 %11, %27, %43;\n\t"
+            "addc.cc.u32 %12, %28, %44;\n\taddc.cc.u32 %13, %29, %45;\n\taddc.cc.u32 %14, %30, %46;\n\t"
+            "addc.u32 %15, %31, %47;" DV_WIDE_OPERANDS(r, a, b));
+        return r;
+    }
+    DV_INL static Wide wide_sub(const Wide& a, const Wide& b) {
+        Wide r;
+        asm("sub.cc.u32 %0, %16, %32;\n\tsubc.cc.u32 %1, %17, %33;\n\tsubc.cc.u32 %2, %18, %34;\n\t"
+            "subc.cc.u32 %3, %19, %35;\n\tsubc.cc.u32 %4, %20, %36;\n\tsubc.cc.u32 %5, %21, %37;\n\t"
+            "subc.cc.u32 %6, %22, %38;\n\tsubc.cc.u32 %7, %23, %39;\n\tsubc.cc.u32 %8, %24, %40;\n\t"
+            "subc.cc.u32 %9, %25, %41;\n\tsubc.cc.u32 %10, %26, %42;\n\tsubc.cc.u32 %11, %27, %43;\n\t"
+            "subc.cc.u32 %12, %28, %44;\n\tsubc.cc.u32 %13, %29, %45;\n\tsubc.cc.u32 %14, %30, %46;\n\t"
+            "subc.u32 %15, %31, %47;" DV_WIDE_OPERANDS(r, a, b));
+        return r;
+    }
+    // A negative t in (-2^255 p, 0) made non-negative by adding 2^255 p.
+    // Differences of up to two products each way qualify: 2 p^2 < 2^255 p.
+    DV_INL static void make_positive(Wide& t) {
+        const uint32_t neg = (uint32_t)((int32_t)t.v[15] >> 31);
+        const uint32_t p[8] = {C::P0, C::P1, C::P2, C::P3, C::P4, C::P5, C::P6, C::P7};
+        uint32_t q[9];  // 2^31 p: words 7..15 of 2^255 p
+        q[0] = (p[0] << 31) & neg;
+#pragma unroll
+        for (int j = 1; j < 8; ++j) q[j] = ((p[j] << 31) | (p[j - 1] >> 1)) & neg;
+        q[8] = (p[7] >> 1) & neg;
+        asm("add.cc.u32 %0, %0, %9;\n\taddc.cc.u32 %1, %1, %10;\n\taddc.cc.u32 %2, %2, %11;\n\t"
+            "addc.cc.u32 %3, %3, %12;\n\taddc.cc.u32 %4, %4, %13;\n\taddc.cc.u32 %5, %5, %14;\n\t"
+            "addc.cc.u32 %6, %6, %15;\n\taddc.cc.u32 %7, %7, %16;\n\taddc.u32 %8, %8, %17;"
+            : "+r"(t.v[7]), "+r"(t.v[8]), "+r"(t.v[9]), "+r"(t.v[10]), "+r"(t.v[11]), "+r"(t.v[12]), "+r"(t.v[13]),
+              "+r"(t.v[14]), "+r"(t.v[15])
+            : "r"(q[0]), "r"(q[1]), "r"(q[2]), "r"(q[3]), "r"(q[4]), "r"(q[5]), "r"(q[6]), "r"(q[7]), "r"(q[8]));
+    }
+    // t / 2^256 mod p for 0 <= t < 2^255 p: the low half is reduced by itself
+    // to at most p + p / 2^32, and with the high half (below p / 2) the sum
+    // stays below 2p.
+    DV_INL static Fp redc(const Wide& w) {
+        constexpr Words N = reduction_words();
+        uint32_t e[8], o[8], t[8];
+        {
+            const uint32_t t0 = w.v[0];
+            asm("mad.lo.cc.u32 %0, %8, %12, %13;\n\tmadc.hi.u32 %1, %8, %12, 0;\n\t"
+                "mul.lo.u32 %2, %9, %12;\n\tmul.hi.u32 %3, %9, %12;\n\t"
+                "mul.lo.u32 %4, %10, %12;\n\tmul.hi.u32 %5, %10, %12;\n\t"
+                "mul.lo.u32 %6, %11, %12;\n\tmul.hi.u32 %7, %11, %12;"
+                : "=&r"(e[0]), "=&r"(e[1]), "=&r"(e[2]), "=&r"(e[3]), "=&r"(e[4]), "=&r"(e[5]), "=&r"(e[6]),
+                  "=&r"(e[7])
+                : "r"(N.v[0]), "r"(N.v[2]), "r"(N.v[4]), "r"(N.v[6]), "r"(t0), "r"(w.v[1]));
+#pragma unroll
+            for (int j = 0; j < 6; ++j) o[j] = w.v[j + 2];
+            o[6] = o[7] = 0;
+            mac4(o, N.v[1], N.v[3], N.v[5], N.v[7], t0);
+        }
+#pragma unroll
+        for (int i = 1; i < 6; ++i) {
+            const uint32_t t0 = e[0];
+            shift_mac4(t, o, e, N.v[1], N.v[3], N.v[5], N.v[7], t0);
+            mac4_top(o, t[7], N.v[0], N.v[2], N.v[4], N.v[6], t0);
+            rotate(e, o, t);
+        }
+        reduce_step(e, o);
+        const uint32_t m = (o[0] + e[1]) * C::INV;
+        shift_mac4(t, o, e, C::P1, C::P3, C::P5, C::P7, m);
+        mac4_top(o, t[7], C::P0, C::P2, C::P4, C::P6, m);
+        rotate(e, o, t);
+        uint32_t q[8];
+        merge(q, e, o);
+        Fp r;
+        asm("add.cc.u32 %0, %8, %16;\n\taddc.cc.u32 %1, %9, %17;\n\taddc.cc.u32 %2, %10, %18;\n\t"
+            "addc.cc.u32 %3, %11, %19;\n\taddc.cc.u32 %4, %12, %20;\n\taddc.cc.u32 %5, %13, %21;\n\t"
+            "addc.cc.u32 %6, %14, %22;\n\taddc.u32 %7, %15, %23;"
+            : "=&r"(r.v[0]), "=&r"(r.v[1]), "=&r"(r.v[2]), "=&r"(r.v[3]), "=&r"(r.v[4]), "=&r"(r.v[5]),
+              "=&r"(r.v[6]), "=&r"(r.v[7])
+            : "r"(q[0]), "r"(q[1]), "r"(q[2]), "r"(q[3]), "r"(q[4]), "r"(q[5]), "r"(q[6]), "r"(q[7]), "r"(w.v[8]),
+              "r"(w.v[9]), "r"(w.v[10]), "r"(w.v[11]), "r"(w.v[12]), "r"(w.v[13]), "r"(w.v[14]), "r"(w.v[15]));
         reduce_once(r.v);
         return r;
     }
+    // Montgomery square: 36 products and the reduction, against a product's 64.
+    DV_INL static Fp sqr_inl(const Fp& a) { return redc(sqr_wide(a)); }
 #ifndef DV_MUL_INLINE
     __device__ __noinline__ static Fp sqr(Fp a) { return sqr_inl(a); }
     // two independent squares in one body, like mul2
@@ -453,6 +500,118 @@ struct __align__(16) Fp {  // 16-byte aligned: global copies move as 128-bit acc
     }
 
   private:
+    struct Words {
+        uint32_t v[8];
+    };
+    // N = (p INV + 1) / 2^32
+    DV_INL static constexpr Words reduction_words() {
+        const uint32_t p[8] = {C::P0, C::P1, C::P2, C::P3, C::P4, C::P5, C::P6, C::P7};
+        Words r{};
+        uint64_t c = 1 + (uint64_t)p[0] * C::INV;  // low word 0
+        for (int i = 1; i < 8; ++i) {
+            c = (c >> 32) + (uint64_t)p[i] * C::INV;
+            r.v[i - 1] = (uint32_t)c;
+        }
+        r.v[7] = (uint32_t)(c >> 32);
+        return r;
+    }
+    // Rows over an accumulator of four register pairs: d = x b, d += x b, d
+    // += x b with the carry out added to top.
+    DV_INL static void mul4(uint32_t* d, uint32_t x0, uint32_t x1, uint32_t x2, uint32_t x3, uint32_t b) {
+        asm("mul.lo.u32 %0, %8, %12;\n\tmul.hi.u32 %1, %8, %12;\n\t"
+            "mul.lo.u32 %2, %9, %12;\n\tmul.hi.u32 %3, %9, %12;\n\t"
+            "mul.lo.u32 %4, %10, %12;\n\tmul.hi.u32 %5, %10, %12;\n\t"
+            "mul.lo.u32 %6, %11, %12;\n\tmul.hi.u32 %7, %11, %12;"
+            : "=&r"(d[0]), "=&r"(d[1]), "=&r"(d[2]), "=&r"(d[3]), "=&r"(d[4]), "=&r"(d[5]), "=&r"(d[6]), "=&r"(d[7])
+            : "r"(x0), "r"(x1), "r"(x2), "r"(x3), "r"(b));
+    }
+    DV_INL static void mac4(uint32_t* d, uint32_t x0, uint32_t x1, uint32_t x2, uint32_t x3, uint32_t b) {
+        asm("mad.lo.cc.u32 %0, %8, %12, %0;\n\tmadc.hi.cc.u32 %1, %8, %12, %1;\n\t"
+            "madc.lo.cc.u32 %2, %9, %12, %2;\n\tmadc.hi.cc.u32 %3, %9, %12, %3;\n\t"
+            "madc.lo.cc.u32 %4, %10, %12, %4;\n\tmadc.hi.cc.u32 %5, %10, %12, %5;\n\t"
+            "madc.lo.cc.u32 %6, %11, %12, %6;\n\tmadc.hi.u32 %7, %11, %12, %7;"
+            : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3]), "+r"(d[4]), "+r"(d[5]), "+r"(d[6]), "+r"(d[7])
+            : "r"(x0), "r"(x1), "r"(x2), "r"(x3), "r"(b));
+    }
+    DV_INL static void mac4_top(uint32_t* d, uint32_t& top, uint32_t x0, uint32_t x1, uint32_t x2, uint32_t x3,
+                                uint32_t b) {
+        asm("mad.lo.cc.u32 %0, %9, %13, %0;\n\tmadc.hi.cc.u32 %1, %9, %13, %1;\n\t"
+            "madc.lo.cc.u32 %2, %10, %13, %2;\n\tmadc.hi.cc.u32 %3, %10, %13, %3;\n\t"
+            "madc.lo.cc.u32 %4, %11, %13, %4;\n\tmadc.hi.cc.u32 %5, %11, %13, %5;\n\t"
+            "madc.lo.cc.u32 %6, %12, %13, %6;\n\tmadc.hi.cc.u32 %7, %12, %13, %7;\n\t"
+            "addc.u32 %8, %8, 0;"
+            : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3]), "+r"(d[4]), "+r"(d[5]), "+r"(d[6]), "+r"(d[7]),
+              "+r"(top)
+            : "r"(x0), "r"(x1), "r"(x2), "r"(x3), "r"(b));
+    }
+    // The shift of T = E + 2^32 O by one limb (the low limb is done with): o
+    // becomes the new E with e[1] added to its low word, whose carry (the
+    // weight of the new O's low word) starts the chain t = x b + (e without two words).
+    DV_INL static void shift_mac4(uint32_t* t, uint32_t* o, const uint32_t* e, uint32_t x0, uint32_t x1, uint32_t x2,
+                                  uint32_t x3, uint32_t b) {
+        asm("add.cc.u32 %8, %8, %14;\n\t"
+            "madc.lo.cc.u32 %0, %9, %13, %15;\n\tmadc.hi.cc.u32 %1, %9, %13, %16;\n\t"
+            "madc.lo.cc.u32 %2, %10, %13, %17;\n\tmadc.hi.cc.u32 %3, %10, %13, %18;\n\t"
+            "madc.lo.cc.u32 %4, %11, %13, %19;\n\tmadc.hi.cc.u32 %5, %11, %13, %20;\n\t"
+            "madc.lo.cc.u32 %6, %12, %13, 0;\n\tmadc.hi.u32 %7, %12, %13, 0;"
+            : "=&r"(t[0]), "=&r"(t[1]), "=&r"(t[2]), "=&r"(t[3]), "=&r"(t[4]), "=&r"(t[5]), "=&r"(t[6]), "=&r"(t[7]),
+              "+r"(o[0])
+            : "r"(x0), "r"(x1), "r"(x2), "r"(x3), "r"(b), "r"(e[1]), "r"(e[2]), "r"(e[3]), "r"(e[4]), "r"(e[5]),
+              "r"(e[6]), "r"(e[7]));
+    }
+    DV_INL static void rotate(uint32_t* e, uint32_t* o, const uint32_t* t) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            e[j] = o[j];
+            o[j] = t[j];
+        }
+    }
+    // One step with the exact multiplier: afterwards e[0] = 0.
+    DV_INL static void reduce_step(uint32_t* e, uint32_t* o) {
+        const uint32_t m = e[0] * C::INV;
+        mac4(o, C::P1, C::P3, C::P5, C::P7, m);
+        mac4_top(e, o[7], C::P0, C::P2, C::P4, C::P6, m);
+    }
+    // r = (E >> 32) + O
+    DV_INL static void merge(uint32_t* r, const uint32_t* e, const uint32_t* o) {
+        asm("add.cc.u32 %0, %8, %16;\n\taddc.cc.u32 %1, %9, %17;\n\taddc.cc.u32 %2, %10, %18;\n\t"
+            "addc.cc.u32 %3, %11, %19;\n\taddc.cc.u32 %4, %12, %20;\n\taddc.cc.u32 %5, %13, %21;\n\t"
+            "addc.cc.u32 %6, %14, %22;\n\taddc.u32 %7, %15, 0;"
+            : "=&r"(r[0]), "=&r"(r[1]), "=&r"(r[2]), "=&r"(r[3]), "=&r"(r[4]), "=&r"(r[5]), "=&r"(r[6]), "=&r"(r[7])
+            : "r"(o[0]), "r"(o[1]), "r"(o[2]), "r"(o[3]), "r"(o[4]), "r"(o[5]), "r"(o[6]), "r"(o[7]), "r"(e[1]),
+              "r"(e[2]), "r"(e[3]), "r"(e[4]), "r"(e[5]), "r"(e[6]), "r"(e[7]));
+    }
+    // K products x[k] m added to the pairs at d, the carry out to top.
+    template <int K>
+    DV_INL static void chain(uint32_t* d, const uint32_t* x, uint32_t m, uint32_t& top) {
+        if constexpr (K == 1)
+            asm("mad.lo.cc.u32 %0, %3, %4, %0;\n\tmadc.hi.cc.u32 %1, %3, %4, %1;\n\taddc.u32 %2, %2, 0;"
+                : "+r"(d[0]), "+r"(d[1]), "+r"(top)
+                : "r"(x[0]), "r"(m));
+        else if constexpr (K == 2)
+            asm("mad.lo.cc.u32 %0, %5, %7, %0;\n\tmadc.hi.cc.u32 %1, %5, %7, %1;\n\t"
+                "madc.lo.cc.u32 %2, %6, %7, %2;\n\tmadc.hi.cc.u32 %3, %6, %7, %3;\n\taddc.u32 %4, %4, 0;"
+                : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3]), "+r"(top)
+                : "r"(x[0]), "r"(x[1]), "r"(m));
+        else if constexpr (K == 3)
+            asm("mad.lo.cc.u32 %0, %7, %10, %0;\n\tmadc.hi.cc.u32 %1, %7, %10, %1;\n\t"
+                "madc.lo.cc.u32 %2, %8, %10, %2;\n\tmadc.hi.cc.u32 %3, %8, %10, %3;\n\t"
+                "madc.lo.cc.u32 %4, %9, %10, %4;\n\tmadc.hi.cc.u32 %5, %9, %10, %5;\n\taddc.u32 %6, %6, 0;"
+                : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3]), "+r"(d[4]), "+r"(d[5]), "+r"(top)
+                : "r"(x[0]), "r"(x[1]), "r"(x[2]), "r"(m));
+        else
+            mac4_top(d, top, x[0], x[1], x[2], x[3], m);
+    }
+    // E + 2^32 O of a 512-bit value
+    DV_INL static Wide combine(const uint32_t* e, const uint32_t* o) {
+        Wide a, b;
+        b.v[0] = 0;
+#pragma unroll
+        for (int j = 0; j < 16; ++j) a.v[j] = e[j];
+#pragma unroll
+        for (int j = 1; j < 16; ++j) b.v[j] = o[j - 1];
+        return wide_add(a, b);
+    }
     // Signed 30-bit-limb numbers of the divstep inverse.
     struct N9 {
         int32_t l[9];
