@@ -3,7 +3,8 @@
 // point at infinity.  Formulas are the a = 0 specialisations of the
 // Explicit-Formulas Database "xyzz" family (madd-2008-s, add-2008-s,
 // dbl-2008-s-1, mdbl-2008-s-1): mixed add 8M+2S, full add 12M+2S,
-// double 6M+3S.  Affine infinity is encoded as (0, 0), which is on neither
+// double 6M+3S, in each of which Y3 = a b - c d takes one reduction for two
+// products.  Affine infinity is encoded as (0, 0), which is on neither
 // curve.
 #pragma once
 #include "field.cuh"
@@ -39,7 +40,7 @@ struct XYZZ {
         const F x2 = F::sqr(a.x);
         const F m = F::add(F::dbl(x2), x2);
         const F x3 = F::sub(F::sqr(m), F::dbl(s));
-        const F y3 = F::sub(F::mul(m, F::sub(s, x3)), F::mul(w, a.y));
+        const F y3 = F::mul_sub(m, F::sub(s, x3), w, a.y);
         return {x3, y3, v, w};
     }
 
@@ -53,7 +54,7 @@ struct XYZZ {
         const F x2 = F::sqr(p.x);
         const F m = F::add(F::dbl(x2), x2);
         const F x3 = F::sub(F::sqr(m), F::dbl(s));
-        const F y3 = F::sub(F::mul(m, F::sub(s, x3)), F::mul(w, p.y));
+        const F y3 = F::mul_sub(m, F::sub(s, x3), w, p.y);
         return {x3, y3, F::mul(v, p.zz), F::mul(w, p.zzz)};
     }
 
@@ -64,10 +65,11 @@ struct XYZZ {
         return inf();
     }
 
-    // p + a with a affine (madd-2008-s).  Over Fq the ten products are
-    // issued as five independent pairs (F::mul2): measured 7 % faster bucket
-    // accumulation; over Fq2, whose products already hold three independent
-    // chains, the plain sequence is faster.
+    // p + a with a affine (madd-2008-s).  Over Fq eight of the ten products are
+    // issued as four independent pairs (F::mul2, F::sqr2): measured 7 % faster
+    // bucket accumulation; over Fq2, whose products already hold three
+    // independent chains, the plain sequence is faster.  Y3's two products
+    // share one reduction (F::mul_sub).
     DV_INL static XYZZ add_affine(const XYZZ& p, const Affine<F>& a) {
         if (a.is_inf()) return p;
         if (p.is_inf()) return from_affine(a);
@@ -82,8 +84,7 @@ struct XYZZ {
             const F ppp = pq.r0, q = pq.r1;
             const F x3 = F::sub(F::sub(sq.r1, ppp), F::dbl(q));
             const auto zs = F::mul2(p.zz, pp, p.zzz, ppp);      // ZZ3, ZZZ3
-            const auto ys = F::mul2(r, F::sub(q, x3), p.y, ppp);
-            return {x3, F::sub(ys.r0, ys.r1), zs.r0, zs.r1};
+            return {x3, F::mul_sub(r, F::sub(q, x3), p.y, ppp), zs.r0, zs.r1};
         } else {
             const F u2 = F::mul(a.x, p.zz);
             const F s2 = F::mul(a.y, p.zzz);
@@ -94,7 +95,7 @@ struct XYZZ {
             const F ppp = F::mul(pp_, pp);
             const F q = F::mul(p.x, pp);
             const F x3 = F::sub(F::sub(F::sqr(r), ppp), F::dbl(q));
-            const F y3 = F::sub(F::mul(r, F::sub(q, x3)), F::mul(p.y, ppp));
+            const F y3 = F::mul_sub(r, F::sub(q, x3), p.y, ppp);
             return {x3, y3, F::mul(p.zz, pp), F::mul(p.zzz, ppp)};
         }
     }
@@ -117,7 +118,7 @@ struct XYZZ {
         const F ppp = F::mul(pp_, pp);
         const F qq = F::mul(u1, pp);
         const F x3 = F::sub(F::sub(F::sqr(r), ppp), F::dbl(qq));
-        const F y3 = F::sub(F::mul(r, F::sub(qq, x3)), F::mul(s1, ppp));
+        const F y3 = F::mul_sub(r, F::sub(qq, x3), s1, ppp);
         return {x3, y3, F::mul(F::mul(p.zz, q.zz), pp), F::mul(F::mul(p.zzz, q.zzz), ppp)};
     }
 
@@ -132,11 +133,9 @@ struct XYZZ {
         const auto ws = F::mul2(u, v, p.x, v);         // W = U V, S = X V
         const F w = ws.r0, s = ws.r1;
         const F m = F::add(F::dbl(vx.r1), vx.r1);
-        const auto mz = F::mul2(m, m, v, p.zz);        // M^2, ZZ3
-        const F x3 = F::sub(mz.r0, F::dbl(s));
-        const auto wy = F::mul2(w, p.y, w, p.zzz);     // W Y, ZZZ3
-        const F y3 = F::sub(F::mul(m, F::sub(s, x3)), wy.r0);
-        return {x3, y3, mz.r1, wy.r1};
+        const F x3 = F::sub(F::sqr(m), F::dbl(s));
+        const auto zs = F::mul2(v, p.zz, w, p.zzz);    // ZZ3, ZZZ3
+        return {x3, F::mul_sub(m, F::sub(s, x3), w, p.y), zs.r0, zs.r1};
     }
     DV_INL static XYZZ add_paired(const XYZZ& p, const XYZZ& q) {
         if (p.is_inf()) return q;
@@ -156,8 +155,7 @@ struct XYZZ {
         const F x3 = F::sub(F::sub(sq.r1, ppp), F::dbl(qq));
         const auto zz = F::mul2(p.zz, q.zz, p.zzz, q.zzz);
         const auto zs = F::mul2(zz.r0, pp, zz.r1, ppp);  // ZZ3, ZZZ3
-        const auto ys = F::mul2(r, F::sub(qq, x3), s.r0, ppp);
-        return {x3, F::sub(ys.r0, ys.r1), zs.r0, zs.r1};
+        return {x3, F::mul_sub(r, F::sub(qq, x3), s.r0, ppp), zs.r0, zs.r1};
     }
 
     // Projective equality without normalisation.

@@ -205,11 +205,14 @@ __global__ void k_scatter(const uint32_t* __restrict__ scalars, uint32_t n, cons
 }
 
 // 4. Balanced accumulation over the sorted list.
-#ifndef DV_ACCUM_MINB
-#define DV_ACCUM_MINB 4
-#endif
+// Resident blocks per SM: four for G1 (128 registers, which its accumulator
+// and the paired products fit but for 250 bytes), two for G2, whose 255
+// registers leave 290 bytes of spills where four blocks' 128 left 2.5 KB
+// (G2 MSM of 2^16 points: 2.24 to 2.03 ms; three blocks 2.12 ms).
 template <class F>
-__global__ void __launch_bounds__(128, DV_ACCUM_MINB) k_accum(const Affine<F>* __restrict__ pts, const uint32_t* __restrict__ sorted,
+constexpr int ACCUM_BLOCKS = sizeof(F) == sizeof(Fq) ? 4 : 2;
+template <class F>
+__global__ void __launch_bounds__(128, ACCUM_BLOCKS<F>) k_accum(const Affine<F>* __restrict__ pts, const uint32_t* __restrict__ sorted,
                                                const uint32_t* __restrict__ offsets, uint32_t nb,
                                                XYZZ<F>* __restrict__ buckets, int* __restrict__ pgid,
                                                XYZZ<F>* __restrict__ ppt) {

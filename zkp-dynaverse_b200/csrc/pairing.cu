@@ -139,34 +139,6 @@ DV_INL Fq shfl_fq(const Fq& a, int src) {
 DV_INL Fq2 shfl2(const Fq2& a, int src) { return {shfl_fq(a.c0, src), shfl_fq(a.c1, src)}; }
 DV_INL int mod6(int x) { return x < 0 ? x + 6 : (x >= 6 ? x - 6 : x); }
 
-// n Fq2 products (Karatsuba, 3 base products each) with their 3n base
-// products issued two at a time (one out-of-line body interleaves the two
-// chains, which a lone warp needs to hide the multiply latency).
-template <int N>
-DV_INL void fq2_mul_n(const Fq2* a, const Fq2* b, Fq2* out) {
-    constexpr int M = 3 * N, G = (M + 1) / 2;
-    Fq x[2 * G], y[2 * G], z[2 * G];
-#pragma unroll
-    for (int i = 0; i < N; ++i) {
-        x[3 * i] = a[i].c0; y[3 * i] = b[i].c0;
-        x[3 * i + 1] = a[i].c1; y[3 * i + 1] = b[i].c1;
-        x[3 * i + 2] = Fq::add(a[i].c0, a[i].c1); y[3 * i + 2] = Fq::add(b[i].c0, b[i].c1);
-    }
-#pragma unroll
-    for (int g = 0; g < G; ++g) {
-        if (2 * g + 1 < M) {
-            const Fq::Pair q = Fq::mul2(x[2 * g], y[2 * g], x[2 * g + 1], y[2 * g + 1]);
-            z[2 * g] = q.r0;
-            z[2 * g + 1] = q.r1;
-        } else {
-            z[2 * g] = Fq::mul(x[2 * g], y[2 * g]);
-        }
-    }
-#pragma unroll
-    for (int i = 0; i < N; ++i)
-        out[i] = {Fq::sub(z[3 * i], z[3 * i + 1]), Fq::sub(Fq::sub(z[3 * i + 2], z[3 * i]), z[3 * i + 1])};
-}
-
 // Products and squares by Karatsuba over Fq4 = Fq2[t]/(t^2 - xi), t = w^3:
 // f = F0 + F1 w + F2 w^2 with F_i = f_i + f_(i+3) t and w^3 = t.  The six
 // Fq4 products of a three-term Karatsuba, one per lane (three Fq2 products
@@ -229,7 +201,8 @@ __device__ __noinline__ Fq2 g_mul(const Fq2& a, const Fq2& b, int k, int base) {
     const Fq4 x = k_operand(a, k, base), y = k_operand(b, k, base);
     const Fq2 xs[3] = {x.r, x.s, Fq2::add(x.r, x.s)}, ys[3] = {y.r, y.s, Fq2::add(y.r, y.s)};
     Fq2 p[3];
-    fq2_mul_n<3>(xs, ys, p);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) p[i] = Fq2::mul(xs[i], ys[i]);
     return k_combine({Fq2::add(p[0], mul_xi(p[1])), Fq2::sub(Fq2::sub(p[2], p[0]), p[1])}, k, base);
 }
 // c = a^2 (the same Karatsuba with Fq4 squares: three Fq2 squares a lane).
@@ -279,7 +252,8 @@ __device__ __noinline__ Fq2 g_mul_line(const Fq2& f, const Fq2& l0, const Fq2& l
     const Fq2 x[3] = {f, shfl2(f, base + mod6(k - 1)), shfl2(f, base + mod6(k - 3))};
     const Fq2 y[3] = {l0, l1, l3};
     Fq2 p[3];
-    fq2_mul_n<3>(x, y, p);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) p[i] = Fq2::mul(x[i], y[i]);
     return Fq2::add(Fq2::add(p[0], k < 1 ? mul_xi(p[1]) : p[1]), k < 3 ? mul_xi(p[2]) : p[2]);
 }
 // f^(q^6): w -> -w.
@@ -327,20 +301,13 @@ struct Tw {
     Fq2 x, y, z;  // Jacobian on the twist
 };
 
-// a b with the two base products a0 b0, a1 b1 issued as a pair.
-DV_INL Fq2 fq2_mul_fast(const Fq2& a, const Fq2& b) {
-    const Fq::Pair p = Fq::mul2(a.c0, b.c0, a.c1, b.c1);
-    const Fq t = Fq::mul(Fq::add(a.c0, a.c1), Fq::add(b.c0, b.c1));
-    return {Fq::sub(p.r0, p.r1), Fq::sub(Fq::sub(t, p.r0), p.r1)};
-}
 DV_INL Fq2 pick(int k, const Fq2& v0, const Fq2& v1, const Fq2& v2, const Fq2& v3, const Fq2& v4, const Fq2& v5) {
     return k == 0 ? v0 : k == 1 ? v1 : k == 2 ? v2 : k == 3 ? v3 : k == 4 ? v4 : v5;
 }
 // Each lane of the group computes one Fq2 product, its operands chosen by
 // k, and gets every lane's product back.
 DV_INL void level(const Fq2& a, const Fq2& b, int base, Fq2* out, int n) {
-    Fq2 p;
-    fq2_mul_n<1>(&a, &b, &p);
+    const Fq2 p = Fq2::mul(a, b);
 #pragma unroll
     for (int j = 0; j < 6; ++j)
         if (j < n) out[j] = shfl2(p, base + j);
@@ -377,7 +344,7 @@ __device__ __noinline__ void dbl_step(Tw& t, const Fq& xp, const Fq& yp, Fq2& l0
 __device__ __noinline__ void add_step(Tw& t, const Fq2& xs, const Fq2& ys, const Fq& xp, const Fq& yp, Fq2& l0,
                                       Fq2& l1, Fq2& l3, int k, int base) {
     Fq2 v[6];
-    const Fq2 zz = fq2_mul_fast(t.z, t.z);
+    const Fq2 zz = Fq2::mul(t.z, t.z);
     level(pick(k, xs, t.z, xs, xs, xs, xs), pick(k, zz, zz, zz, zz, zz, zz), base, v, 2);
     const Fq2 h = Fq2::sub(v[0], t.x), zh = Fq2::add(t.z, h);
     level(pick(k, ys, h, zh, h, h, h), pick(k, v[1], h, zh, h, h, h), base, v, 3);
@@ -441,7 +408,7 @@ __device__ __noinline__ void prep_dbl(Tw& t, Line& l, int k, int base) {
 }
 __device__ __noinline__ void prep_add(Tw& t, const Fq2& xs, const Fq2& ys, Line& l, int k, int base) {
     Fq2 v[6];
-    const Fq2 zz = fq2_mul_fast(t.z, t.z);
+    const Fq2 zz = Fq2::mul(t.z, t.z);
     level(pick(k, xs, t.z, xs, xs, xs, xs), pick(k, zz, zz, zz, zz, zz, zz), base, v, 2);
     const Fq2 h = Fq2::sub(v[0], t.x), zh = Fq2::add(t.z, h);
     level(pick(k, ys, h, zh, h, h, h), pick(k, v[1], h, zh, h, h, h), base, v, 3);
@@ -531,8 +498,7 @@ DV_INL void scale_two(const Line& x, const G1A& p, bool one_x, const Line& y, co
 __device__ __noinline__ Fq2 g_line_line(const SLine& a, const SLine& b, int k, int base) {
     const Fq2 x = k == 0 ? a.l0 : k == 1 ? a.l1 : k == 2 ? a.l3 : Fq2::add(k == 5 ? a.l1 : a.l0, k == 3 ? a.l1 : a.l3);
     const Fq2 y = k == 0 ? b.l0 : k == 1 ? b.l1 : k == 2 ? b.l3 : Fq2::add(k == 5 ? b.l1 : b.l0, k == 3 ? b.l1 : b.l3);
-    Fq2 p;
-    fq2_mul_n<1>(&x, &y, &p);
+    const Fq2 p = Fq2::mul(x, y);
     const Fq2 m = shfl2(p, base + (k == 1 ? 3 : k == 2 ? 1 : k == 3 ? 4 : k == 4 ? 5 : 0));
     const Fq2 p0 = shfl2(p, base), p1 = shfl2(p, base + 1), p2 = shfl2(p, base + 2);
     const Fq2 d = Fq2::sub(Fq2::sub(m, k == 4 ? p1 : p0), k == 1 ? p1 : p2);
