@@ -68,6 +68,7 @@
 #include <set>
 #include <string>
 #include <thread>
+#include <unordered_map>
 #include <unordered_set>
 #include <vector>
 
@@ -1337,7 +1338,14 @@ public:
         run([&] { id = open_impl(pid, pub, witness, proof); });
         return id;
     }
+    // Refused while any request of the session is unfinished when the call is
+    // made, queued or in a running batch: which of the two it is depends on
+    // how soon the worker looks at its queue.
     void close_session(uint64_t id) {
+        {
+            std::lock_guard<std::mutex> lk(mu_);
+            if (unfinished_.count(id)) throw InvalidArgument("session has pending requests");
+        }
         run([&] {
             std::lock_guard<std::mutex> lk(mu_);
             auto it = sessions_.find(id);
@@ -1383,6 +1391,7 @@ public:
         if (!sessions_.count(session)) throw InvalidArgument("unknown session");
         r.ticket = next_ticket_++;
         outcomes_[r.ticket];
+        ++unfinished_[session];
         queue_.push_back(std::move(r));
         cv_.notify_all();
         return queue_.back().ticket;
@@ -1497,6 +1506,8 @@ private:
                 o.res.batch_requests = (uint32_t)batch.size();
                 o.res.batch_id = (uint32_t)stat_batches_;
                 o.ready = true;
+                const auto u = unfinished_.find(batch[r].session);
+                if (--u->second == 0) unfinished_.erase(u);
             }
             stat_requests_ += batch.size();
             stat_batches_++;
@@ -1570,6 +1581,7 @@ private:
     std::map<uint64_t, std::unique_ptr<Params>> params_;
     std::map<uint64_t, std::unique_ptr<Session>> sessions_;
     std::map<uint64_t, Outcome> outcomes_;
+    std::unordered_map<uint64_t, uint32_t> unfinished_;  // requests without an outcome, per session
     uint64_t next_id_ = 1, next_ticket_ = 1;
     uint64_t stat_requests_ = 0, stat_batches_ = 0, stat_largest_ = 0, stat_busy_ns_ = 0, stat_sparse_ = 0,
              stat_rebuilds_ = 0, stat_launches_ = 0;
