@@ -203,3 +203,20 @@ def test_multi_miller_loop_in_large_batches(backend, oracle):
     sub = offsets[m]
     assert backend.pairing_check(g1[:64 * sub], g2[:128 * sub], offsets[:m + 1]) == \
         oracle.pairing_check(g1[:64 * sub], g2[:128 * sub], offsets[:m + 1])
+
+
+@pytest.mark.parametrize("n", [1, 3, 4, 5, 1184, 1185, 1191])
+def test_lane_group_layouts(backend, oracle, n):
+    """A group takes a warp up to 1184 groups a call and half a warp beyond,
+    four or eight groups a block: GT elements of n pairs with distinct G2
+    points on both sides of these edges against the oracle (a sample), and
+    n one-term equations over two repeated G2 points, every third one trivial."""
+    sa, sb = oracle.uniform_fr(5301, n), oracle.uniform_fr(5302, n)
+    g1, g2 = oracle.fixed_base_g1(sa), oracle.fixed_base_g2(sb)
+    gt = backend.pairing(g1, g2)
+    for i in sorted({0, 1, n // 2, n - 2, n - 1} & set(range(n))):
+        assert gt[384 * i:384 * i + 384] == oracle.pairing(g1[64 * i:64 * i + 64], g2[128 * i:128 * i + 128]), i
+    trivial = [i % 3 == 1 for i in range(n)]
+    p = b"".join(bytes(64) if t else g1[64 * i:64 * i + 64] for i, t in enumerate(trivial))
+    q = b"".join(g2[:128] if i % 2 else g2[-128:] for i in range(n))
+    assert backend.pairing_check(p, q, list(range(n + 1))) == trivial

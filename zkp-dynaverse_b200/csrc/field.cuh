@@ -306,6 +306,13 @@ struct __align__(16) Fp {  // 16-byte aligned: global copies move as 128-bit acc
     // to at most p + p / 2^32, and with the high half (below p / 2) the sum
     // stays below 2p.
     DV_INL static Fp redc(const Wide& w) {
+        Fp r = redc_raw(w);
+        reduce_once(r.v);
+        return r;
+    }
+    // The same without the last subtraction, for a high half of up to 4.27 p
+    // (the sum then stays below 2^256 = 5.29 p).
+    DV_INL static Fp redc_raw(const Wide& w) {
         constexpr Words N = reduction_words();
         uint32_t e[8], o[8], t[8];
         {
@@ -344,7 +351,6 @@ struct __align__(16) Fp {  // 16-byte aligned: global copies move as 128-bit acc
               "=&r"(r.v[6]), "=&r"(r.v[7])
             : "r"(q[0]), "r"(q[1]), "r"(q[2]), "r"(q[3]), "r"(q[4]), "r"(q[5]), "r"(q[6]), "r"(q[7]), "r"(w.v[8]),
               "r"(w.v[9]), "r"(w.v[10]), "r"(w.v[11]), "r"(w.v[12]), "r"(w.v[13]), "r"(w.v[14]), "r"(w.v[15]));
-        reduce_once(r.v);
         return r;
     }
     // Montgomery square: 36 products and the reduction, against a product's 64.
@@ -386,6 +392,31 @@ struct __align__(16) Fp {  // 16-byte aligned: global copies move as 128-bit acc
             : "r"(a.v[0]), "r"(a.v[1]), "r"(a.v[2]), "r"(a.v[3]), "r"(a.v[4]), "r"(a.v[5]), "r"(a.v[6]),
               "r"(a.v[7]), "r"(b.v[0]), "r"(b.v[1]), "r"(b.v[2]), "r"(b.v[3]), "r"(b.v[4]), "r"(b.v[5]),
               "r"(b.v[6]), "r"(b.v[7]));
+        return r;
+    }
+
+    // a - b modulo 2^256
+    DV_INL static Fp sub_raw(const Fp& a, const Fp& b) {
+        Fp r;
+        asm("sub.cc.u32 %0, %8, %16;\n\t"
+            "subc.cc.u32 %1, %9, %17;\n\t"
+            "subc.cc.u32 %2, %10, %18;\n\t"
+            "subc.cc.u32 %3, %11, %19;\n\t"
+            "subc.cc.u32 %4, %12, %20;\n\t"
+            "subc.cc.u32 %5, %13, %21;\n\t"
+            "subc.cc.u32 %6, %14, %22;\n\t"
+            "subc.u32 %7, %15, %23;"
+            : "=r"(r.v[0]), "=r"(r.v[1]), "=r"(r.v[2]), "=r"(r.v[3]), "=r"(r.v[4]), "=r"(r.v[5]),
+              "=r"(r.v[6]), "=r"(r.v[7])
+            : "r"(a.v[0]), "r"(a.v[1]), "r"(a.v[2]), "r"(a.v[3]), "r"(a.v[4]), "r"(a.v[5]), "r"(a.v[6]),
+              "r"(a.v[7]), "r"(b.v[0]), "r"(b.v[1]), "r"(b.v[2]), "r"(b.v[3]), "r"(b.v[4]), "r"(b.v[5]),
+              "r"(b.v[6]), "r"(b.v[7]));
+        return r;
+    }
+    DV_INL static Fp modulus() {
+        Fp r;
+        r.v[0] = C::P0; r.v[1] = C::P1; r.v[2] = C::P2; r.v[3] = C::P3;
+        r.v[4] = C::P4; r.v[5] = C::P5; r.v[6] = C::P6; r.v[7] = C::P7;
         return r;
     }
 

@@ -4,20 +4,18 @@
 // PairingChecks::equal / equal_prepared / product_equal reduce one equation
 // to prod_k e(P_k, Q_k) = 1 (right-hand G1 points negated by the caller),
 // computed by Bn254::multi_miller_loop and final_exponentiation.  Here a
-// launch takes many equations: a group of six lanes runs the Miller loop of
+// launch takes many equations: a group of lanes runs the Miller loop of
 // one term (or, with prepared G2 points in large batches, the multi-Miller
 // loop of one equation), then a group per equation multiplies its terms'
 // values and runs the final exponentiation.  The reference's native Miller probe
 // (native/include/dynaverse_bn254_miller.h) is a diagnostic of line traces
 // and is not reproduced.
 //
-// Fq12 = Fq2[w]/(w^6 - xi), xi = 9 + u, held by six lanes: lane k owns the
-// coefficient of w^k.  A product is a three-term Karatsuba over
-// Fq4 = Fq2[w^3], one Fq4 product (three Fq2 products) per lane from
-// shuffled operands; a square the same with Fq4 squares; the sparse line
-// product is c_k = sum_i f_i l_(k-i) over the line's three coefficients,
-// three Fq2 products per lane; the q-power Frobenius
-// is conj(a_k) xi^(k(q-1)/6) per lane; f^(q^6) negates the odd lanes.  The
+// Fq12 = Fq2[w]/(w^6 - xi), xi = 9 + u, held by twelve lanes, one component
+// each (see "lane groups"): products, squares and the sparse line product
+// c_k = sum_i f_i l_(k-i) are sums of base products per lane with one
+// reduction; the q-power Frobenius is conj(a_k) xi^(k(q-1)/6) per lane;
+// f^(q^6) negates the odd coefficients.  The
 // serialised GT element uses the tower Fq12 = Fq6[w]/(w^2 - v), Fq6 =
 // Fq2[v]/(v^3 - xi), v = w^2: c0 = (w^0, w^2, w^4), c1 = (w^1, w^3, w^5).
 //
@@ -122,261 +120,347 @@ __device__ __noinline__ Fq6 f6_inv(const Fq6& a) {
 }
 
 // ------------------------------------------------------------------ lane groups
-// One Fq12 lives in a group of GL = 6 lanes: lane k holds the Fq2
-// coefficient of w^k (w^6 = xi).  A warp holds 5 groups (lanes 30, 31 run
-// along on copies and write nothing); every group in a warp executes the
-// same instruction stream, so the shuffles below always see full warps.
+// One Fq12 lives in a group of 16 lanes, twelve of them at work: lane 2k + c
+// holds component c of the Fq2 coefficient of w^k.  Lanes 12 to 15 run along
+// as copies of lanes 0 to 3 and write nothing.  The operands of a product go
+// through shared memory (A plain; B with xi B and the negated second
+// components beside it), and every lane sums the products of its component at
+// 512 bits and reduces once: schoolbook rows with one reduction are fewer
+// multiply-adds a lane than Karatsuba products reduced one by one, and leave
+// no additions between lanes.
+//
+// H = 2 gives a group the whole warp: lanes 16 to 31 take the products with
+// the second components of A, and the two half sums meet in one shuffle.  A
+// group then needs 456 multiply-adds a lane for a product against 840 with
+// H = 1 and two groups a warp.  These kernels are chains of dependent
+// products, so H = 2 is taken while a call's groups leave the GPU's warp
+// slots free, H = 1 (a tenth less work a group) beyond that.
+//
+// Bounds: a sum of up to 12 products of residues is below 12 p^2 < 2^511; its
+// reduction is below 3.3 p, with 2 p added beforehand 5.27 p, and 2^256 is
+// 5.29 p.
 constexpr unsigned FULL = 0xffffffffu;
-constexpr int GL = 6;
-constexpr int GROUPS_PER_WARP = 5;
+constexpr int THREADS = 128;
+template <int H>
+constexpr int GROUPS_PER_BLOCK = THREADS / (16 * H);
+// Shared memory in Fq units: the multiples 0..9 of q, then per group
+// A (6 coefficients and a zero one), B (per coefficient: b0, b1, -b1 and the
+// same of xi b) and V (the products of a level).
+constexpr int SM_MULT = 10, SM_A = 0, SM_B = 14, SM_V = 50, SM_GROUP = 62;
+template <int H>
+constexpr size_t SM_BYTES = sizeof(Fq) * (SM_MULT + SM_GROUP * GROUPS_PER_BLOCK<H>);
+extern __shared__ uint4 pairing_sm[];
+DV_INL Fq* sm(int i) { return reinterpret_cast<Fq*>(pairing_sm) + i; }
 
-DV_INL Fq shfl_fq(const Fq& a, int src) {
+struct Lane {
+    int k, c, h, at;  // coefficient, component, half; the group's place in shared memory
+    bool writes;      // not a copy
+    uint64_t group;   // global group index
+};
+// Also fills the block's tables; ends with a block barrier.
+template <int H>
+DV_INL Lane lane_setup() {
+    const int l = threadIdx.x & 31, j = l & 15, jj = j < 12 ? j : j - 12;
+    const int slot = (int)(threadIdx.x >> 5) * (2 / H) + (H == 1 ? l >> 4 : 0);
+    Lane g;
+    g.k = jj >> 1;
+    g.c = jj & 1;
+    g.h = H == 2 ? l >> 4 : 0;
+    g.at = SM_MULT + SM_GROUP * slot;
+    g.writes = j < 12 && g.h == 0;
+    g.group = (uint64_t)blockIdx.x * GROUPS_PER_BLOCK<H> + slot;
+    if (threadIdx.x < SM_MULT) {
+        Fq m = Fq::zero();
+        for (int i = 0; i < (int)threadIdx.x; ++i) m = Fq::add_raw(m, Fq::modulus());
+        *sm(threadIdx.x) = m;
+    }
+    if (j < 2) *sm(g.at + SM_A + 12 + j) = Fq::zero();
+    __syncthreads();
+    return g;
+}
+DV_INL Fq shfl_xor_fq(const Fq& a, int m) {
     Fq r;
 #pragma unroll
-    for (int w = 0; w < 8; ++w) r.v[w] = __shfl_sync(FULL, a.v[w], src);
+    for (int w = 0; w < 8; ++w) r.v[w] = __shfl_xor_sync(FULL, a.v[w], m);
     return r;
 }
-DV_INL Fq2 shfl2(const Fq2& a, int src) { return {shfl_fq(a.c0, src), shfl_fq(a.c1, src)}; }
-DV_INL int mod6(int x) { return x < 0 ? x + 6 : (x >= 6 ? x - 6 : x); }
-
-// Products and squares by Karatsuba over Fq4 = Fq2[t]/(t^2 - xi), t = w^3:
-// f = F0 + F1 w + F2 w^2 with F_i = f_i + f_(i+3) t and w^3 = t.  The six
-// Fq4 products of a three-term Karatsuba, one per lane (three Fq2 products
-// each, 18 for the group against 36 for the schoolbook form):
-//   lanes 0, 1, 2:  m_i = A_i B_i;
-//   lanes 3, 4, 5:  m12 = (A1 + A2)(B1 + B2), m01 = (A0 + A1)(B0 + B1), m02 = (A0 + A2)(B0 + B2);
-// and C0 = m0 + t (m12 - m1 - m2), C1 = m01 - m0 - m1 + t m2,
-// C2 = m02 - m0 - m2 + m1, C_i = c_i + c_(i+3) t.
-struct Fq4 {
-    Fq2 r, s;  // r + s t
-};
-DV_INL Fq4 shfl4(const Fq4& a, int src) { return {shfl2(a.r, src), shfl2(a.s, src)}; }
-DV_INL Fq4 add4(const Fq4& a, const Fq4& b) { return {Fq2::add(a.r, b.r), Fq2::add(a.s, b.s)}; }
-DV_INL Fq4 sub4(const Fq4& a, const Fq4& b) { return {Fq2::sub(a.r, b.r), Fq2::sub(a.s, b.s)}; }
-
-// Lane k's Karatsuba operand from the group's coefficients: A_k for k < 3,
-// the pair sums A1 + A2, A0 + A1, A0 + A2 on lanes 3, 4, 5.  After the
-// rotations by 1, 2 and 3 lanes, lane j holds f_j + f_(j+1) and
-// f_j + f_(j+2); lanes 3..5 fetch their two halves from lanes (1, 4),
-// (0, 3) and (3, 0), each source lane publishing the one sum asked of it.
-DV_INL Fq4 k_operand(const Fq2& a, int k, int base) {
-    const Fq2 a1 = shfl2(a, base + mod6(k + 1)), a2 = shfl2(a, base + mod6(k + 2));
-    const Fq2 a3 = shfl2(a, base + mod6(k + 3));
-    const Fq2 s1 = Fq2::add(a, a1), s2 = Fq2::add(a, a2);
-    const Fq2 h0 = shfl2(k == 3 ? s2 : s1, base + (k == 3 ? 1 : k == 4 ? 0 : k == 5 ? 3 : k));
-    const Fq2 h1 = shfl2(k == 0 ? s2 : s1, base + (k == 3 ? 4 : k == 4 ? 3 : k == 5 ? 0 : k));
-    if (k < 3) return {a, a3};
-    return k == 5 ? Fq4{h1, h0} : Fq4{h0, h1};
-}
-// Lane k's coefficient of the product from the six Fq4 products m (one per
-// lane): lane i < 3 forms C_i = U + t V from its own m_i, the pair product
-// on lane i + 3 and the other two m_j; lane i + 3 takes the t part of C_i.
-DV_INL Fq2 k_combine(const Fq4& m, int k, int base) {
-    const int i = k < 3 ? k : k - 3;
-    const Fq4 q = shfl4(m, base + mod6(k + 3));
-    const Fq4 n1 = shfl4(m, base + (i == 2 ? 0 : i + 1));
-    const Fq4 n2 = shfl4(m, base + (i == 0 ? 2 : i - 1));
-    const Fq4 t = sub4(sub4(q, n1), n2);
-    // i = 0: U = m0, V = q - n1 - n2; i = 1: U = q - m1 - n0 = t + n2 - m1 (n2 = m0, n1 = m2),
-    // V = n1; i = 2: U = q - m2 - m0 + m1 = t + 2 n2 - m2 (n1 = m0, n2 = m1), V = 0.
-    const Fq4 w = i == 1 ? n1 : add4(n2, n2);
-    const Fq4 u = i == 0 ? m : sub4(add4(t, w), m);
-    const Fq2 vr = i == 0 ? t.r : (i == 1 ? n1.r : Fq2::zero());
-    const Fq2 vs = i == 0 ? t.s : (i == 1 ? n1.s : Fq2::zero());
-    const Fq2 cr = Fq2::add(u.r, mul_xi(vs)), cs = Fq2::add(u.s, vr);
-    const Fq2 hi = shfl2(cs, base + mod6(k + 3));
-    return k < 3 ? cr : hi;
-}
-// x^2 for three Fq2 values, (c0 + c1)(c0 - c1) + 2 c0 c1 u each, the six
-// base products in pairs.
-DV_INL void fq2_sqr_3(const Fq2* a, Fq2* out) {
+DV_INL Fq dbl_raw(const Fq& a, int by = 1) {
+    Fq r;
+    r.v[0] = a.v[0] << by;
 #pragma unroll
-    for (int i = 0; i < 3; ++i) {
-        const Fq::Pair p = Fq::mul2(Fq::add(a[i].c0, a[i].c1), Fq::sub(a[i].c0, a[i].c1), a[i].c0, a[i].c1);
-        out[i] = {p.r0, Fq::dbl(p.r1)};
+    for (int w = 1; w < 8; ++w) r.v[w] = __funnelshift_l(a.v[w - 1], a.v[w], by);
+    return r;
+}
+DV_INL Fq neg_raw(const Fq& a) { return Fq::sub_raw(Fq::modulus(), a); }  // q - a (q for 0)
+// v - (a multiple of q) in [0, q) for v < 10 q with top = v >> 252: the
+// quotient 21 top / 64 is never too large and at most one too small.
+DV_INL Fq reduce_top(const Fq& low, uint32_t top) {
+    Fq r = Fq::sub_raw(low, *sm((int)((top * 21u) >> 6)));
+    Fq::reduce_once(r.v);
+    return r;
+}
+// This lane's component of xi b: 9 b0 - b1 and 9 b1 + b0.
+DV_INL Fq xi_part(const Fq& b, int c) {
+    const Fq other = shfl_xor_fq(b, 1);
+    const Fq q = c ? other : neg_raw(other);
+    const Fq s = dbl_raw(b, 3);
+    uint32_t top = b.v[7] >> 29;
+    Fq r;
+    asm("add.cc.u32 %0, %9, %17;\n\taddc.cc.u32 %1, %10, %18;\n\taddc.cc.u32 %2, %11, %19;\n\t"
+        "addc.cc.u32 %3, %12, %20;\n\taddc.cc.u32 %4, %13, %21;\n\taddc.cc.u32 %5, %14, %22;\n\t"
+        "addc.cc.u32 %6, %15, %23;\n\taddc.cc.u32 %7, %16, %24;\n\taddc.u32 %8, %8, 0;"
+        : "=&r"(r.v[0]), "=&r"(r.v[1]), "=&r"(r.v[2]), "=&r"(r.v[3]), "=&r"(r.v[4]), "=&r"(r.v[5]), "=&r"(r.v[6]),
+          "=&r"(r.v[7]), "+r"(top)
+        : "r"(s.v[0]), "r"(s.v[1]), "r"(s.v[2]), "r"(s.v[3]), "r"(s.v[4]), "r"(s.v[5]), "r"(s.v[6]), "r"(s.v[7]),
+          "r"(b.v[0]), "r"(b.v[1]), "r"(b.v[2]), "r"(b.v[3]), "r"(b.v[4]), "r"(b.v[5]), "r"(b.v[6]), "r"(b.v[7]));
+    asm("add.cc.u32 %0, %0, %9;\n\taddc.cc.u32 %1, %1, %10;\n\taddc.cc.u32 %2, %2, %11;\n\t"
+        "addc.cc.u32 %3, %3, %12;\n\taddc.cc.u32 %4, %4, %13;\n\taddc.cc.u32 %5, %5, %14;\n\t"
+        "addc.cc.u32 %6, %6, %15;\n\taddc.cc.u32 %7, %7, %16;\n\taddc.u32 %8, %8, 0;"
+        : "+r"(r.v[0]), "+r"(r.v[1]), "+r"(r.v[2]), "+r"(r.v[3]), "+r"(r.v[4]), "+r"(r.v[5]), "+r"(r.v[6]),
+          "+r"(r.v[7]), "+r"(top)
+        : "r"(q.v[0]), "r"(q.v[1]), "r"(q.v[2]), "r"(q.v[3]), "r"(q.v[4]), "r"(q.v[5]), "r"(q.v[6]), "r"(q.v[7]));
+    return reduce_top(r, (top << 4) | (r.v[7] >> 28));
+}
+// Staging of this lane's components (a barrier must stand before, after the
+// last reads, and one after, before the next).
+DV_INL void put_a(const Lane& g, const Fq& a) {
+    if (g.writes) *sm(g.at + SM_A + 2 * g.k + g.c) = a;
+}
+DV_INL void put_b(const Lane& g, const Fq& b, const Fq& xb) {
+    if (!g.writes) return;
+    Fq* s = sm(g.at + SM_B + 6 * g.k);
+    s[g.c] = b;
+    s[3 + g.c] = xb;
+    if (g.c) {
+        s[2] = neg_raw(b);
+        s[5] = neg_raw(xb);
     }
 }
-// c = a b.
-__device__ __noinline__ Fq2 g_mul(const Fq2& a, const Fq2& b, int k, int base) {
-    const Fq4 x = k_operand(a, k, base), y = k_operand(b, k, base);
-    const Fq2 xs[3] = {x.r, x.s, Fq2::add(x.r, x.s)}, ys[3] = {y.r, y.s, Fq2::add(y.r, y.s)};
-    Fq2 p[3];
+DV_INL Fq::Wide wide_zero() {
+    Fq::Wide r;
 #pragma unroll
-    for (int i = 0; i < 3; ++i) p[i] = Fq2::mul(xs[i], ys[i]);
-    return k_combine({Fq2::add(p[0], mul_xi(p[1])), Fq2::sub(Fq2::sub(p[2], p[0]), p[1])}, k, base);
+    for (int w = 0; w < 16; ++w) r.v[w] = 0;
+    return r;
 }
-// c = a^2 (the same Karatsuba with Fq4 squares: three Fq2 squares a lane).
-__device__ __noinline__ Fq2 g_sqr(const Fq2& a, int k, int base) {
-    const Fq4 x = k_operand(a, k, base);
-    const Fq2 xs[3] = {x.r, x.s, Fq2::add(x.r, x.s)};
-    Fq2 p[3];
-    fq2_sqr_3(xs, p);
-    return k_combine({Fq2::add(p[0], mul_xi(p[1])), Fq2::sub(Fq2::sub(p[2], p[0]), p[1])}, k, base);
+// The sum over both halves (H = 2).
+template <int H>
+DV_INL Fq::Wide whole_sum(const Fq::Wide& a) {
+    if constexpr (H == 1) {
+        return a;
+    } else {
+        Fq::Wide o;
+#pragma unroll
+        for (int w = 0; w < 16; ++w) o.v[w] = __shfl_xor_sync(FULL, a.v[w], 16);
+        return Fq::wide_add(a, o);
+    }
+}
+DV_INL Fq redc_large(const Fq::Wide& t) {
+    const Fq r = Fq::redc_raw(t);
+    return reduce_top(r, r.v[7] >> 28);
+}
+// This lane's component of A_i B_j (xi B_j with v): its part of the two
+// base products added to acc.
+template <int H>
+DV_INL void term(Fq::Wide& acc, const Lane& g, const Fq* a, const Fq* b, int dbl) {
+    const int second = g.c ? 0 : 2;  // b0 for component 1, -b1 for component 0
+    if constexpr (H == 2) {
+        acc = Fq::wide_add(acc, Fq::mul_wide(dbl_raw(a[g.h], dbl), b[g.h ? second : g.c]));
+    } else {
+        acc = Fq::wide_add(acc, Fq::mul_wide(dbl_raw(a[0], dbl), b[g.c]));
+        acc = Fq::wide_add(acc, Fq::mul_wide(dbl_raw(a[1], dbl), b[second]));
+    }
+}
+// The staged product A B (six terms), A B for A with the coefficients of a
+// line (w^0, w^1, w^3: three terms), or the square of the element staged as
+// both (pairs i <= j with i + j = k modulo 6, doubled unless i = j: four terms
+// for even k, three for odd k).
+enum DotKind { DOT_FULL, DOT_LINE, DOT_SQUARE };
+template <int H, DotKind KIND>
+__device__ __noinline__ Fq g_dot(Lane g) {
+    Fq::Wide acc = wide_zero();
+    constexpr int TERMS = KIND == DOT_FULL ? 6 : KIND == DOT_LINE ? 3 : 4;
+#pragma unroll 1
+    for (int t = 0; t < TERMS; ++t) {
+        int i, j, xi, dbl = 0;
+        if constexpr (KIND == DOT_SQUARE) {
+            i = (g.k >> 1) - t;
+            if (i < 0) i += 6;
+            j = g.k - i;
+            if (j < 0) j += 6;
+            xi = i + j >= 6;
+            dbl = i != j;
+            if (t == 3 && (g.k & 1)) i = 6;  // the zero coefficient
+        } else {
+            i = KIND == DOT_LINE && t == 2 ? 3 : t;
+            j = g.k - i;
+            xi = j < 0;
+            if (xi) j += 6;
+        }
+        term<H>(acc, g, sm(g.at + SM_A + 2 * i), sm(g.at + SM_B + 6 * j + 3 * xi), dbl);
+    }
+    return redc_large(whole_sum<H>(acc));
+}
+template <int H>
+DV_INL Fq g_mul_staged(const Lane& g, const Fq& a, const Fq& b, const Fq& xb) {
+    __syncwarp();
+    put_a(g, a);
+    put_b(g, b, xb);
+    __syncwarp();
+    return g_dot<H, DOT_FULL>(g);
+}
+template <int H>
+DV_INL Fq g_mul(const Lane& g, const Fq& a, const Fq& b) {
+    return g_mul_staged<H>(g, a, b, xi_part(b, g.c));
+}
+template <int H>
+DV_INL Fq g_sqr(const Lane& g, const Fq& a) {
+    const Fq xa = xi_part(a, g.c);
+    __syncwarp();
+    put_a(g, a);
+    put_b(g, a, xa);
+    __syncwarp();
+    return g_dot<H, DOT_SQUARE>(g);
+}
+// f (l0 + l1 w + l3 w^3), this lane's component of the line on lanes k = 0, 1, 3.
+template <int H>
+DV_INL Fq g_mul_line(const Lane& g, const Fq& f, const Fq& line) {
+    const Fq xf = xi_part(f, g.c);
+    __syncwarp();
+    put_a(g, line);
+    put_b(g, f, xf);
+    __syncwarp();
+    return g_dot<H, DOT_LINE>(g);
 }
 // Square of an element of the cyclotomic subgroup (every value after the
 // easy part of the final exponentiation), by Granger and Scott ("Faster
 // squaring in the cyclotomic subgroup of sixth degree extensions", PKC
 // 2010): with A_i = f_i + f_(i+3) t over Fq4 = Fq2[t]/(t^2 - xi), t = w^3,
 //   f^2 = (3 A0^2 - 2 conj A0) + (3 t A2^2 + 2 conj A1) w + (3 A1^2 - 2 conj A2) w^2.
-// Lane j < 3 squares a_j = f_j and b_j = f_(j+3), lane j + 3 squares
-// a_j + b_j; A^2 = (a^2 + xi b^2) + ((a + b)^2 - a^2 - b^2) t.
-__device__ __noinline__ Fq2 g_cyc_sqr(const Fq2& f, int k, int base) {
-    const int j = k < 3 ? k : k - 3;
-    const Fq2 a = shfl2(f, base + j), b = shfl2(f, base + j + 3);
-    const Fq2 u = k < 3 ? a : Fq2::add(a, b), v = k < 3 ? b : u;
-    // u^2, v^2: (c0 + c1)(c0 - c1) and c0 c1 of each, four base products in two pairs
-    const Fq::Pair p0 = Fq::mul2(Fq::add(u.c0, u.c1), Fq::sub(u.c0, u.c1), Fq::add(v.c0, v.c1), Fq::sub(v.c0, v.c1));
-    const Fq::Pair p1 = Fq::mul2(u.c0, u.c1, v.c0, v.c1);
-    const Fq2 x = {p0.r0, Fq::dbl(p1.r0)}, y = {p0.r1, Fq::dbl(p1.r1)};
-    Fq2 sa[3], sb[3], sab[3];
-#pragma unroll
-    for (int m = 0; m < 3; ++m) {
-        sa[m] = shfl2(x, base + m);
-        sb[m] = shfl2(y, base + m);
-        sab[m] = shfl2(x, base + 3 + m);
+// A^2 = (a^2 + xi b^2) + 2 a b t for A = a + b t: lanes k = 0, 2, 4 sum
+// a a + b (xi b), lanes 3, 5 sum 2 a b, lane 1 sums 2 a (xi b).  Three
+// products a lane with H = 1 (a a by (a0 + a1)(a0 - a1) or 2 a0 a1), two
+// with H = 2; three times the sum and the linear term join before the one reduction.
+template <int H>
+__device__ __noinline__ Fq g_cyc_sqr(Fq f, Lane g) {
+    const Fq xf = xi_part(f, g.c);
+    __syncwarp();
+    put_a(g, f);
+    put_b(g, f, xf);
+    __syncwarp();
+    const int m = g.k == 0 || g.k == 3 ? 0 : (g.k == 2 || g.k == 5 ? 1 : 2);
+    const bool real = !(g.k & 1) && g.k != 3;
+    const Fq* a = sm(g.at + SM_A + 2 * m);
+    const Fq* a3 = sm(g.at + SM_A + 2 * (m + 3));
+    const Fq* b = sm(g.at + SM_B + 6 * m);
+    const Fq* b3 = sm(g.at + SM_B + 6 * (m + 3));
+    const int second = g.c ? 0 : 2;
+    Fq::Wide acc;
+    if constexpr (H == 2) {
+        const int sel = g.h ? second : g.c;
+        const Fq x = real ? a[g.h] : dbl_raw(a[g.h]);
+        acc = Fq::mul_wide(x, real ? b[sel] : b3[sel + (g.k == 1 ? 3 : 0)]);
+        const Fq y = real ? a3[g.h] : Fq::zero();
+        acc = Fq::wide_add(acc, Fq::mul_wide(y, b3[3 + sel]));
+    } else {
+        const Fq a0 = a[0], a1 = a[1];
+        const int xi = real || g.k == 1 ? 3 : 0;
+        acc = Fq::mul_wide(real ? a3[0] : dbl_raw(a0), b3[xi + g.c]);
+        acc = Fq::wide_add(acc, Fq::mul_wide(real ? a3[1] : dbl_raw(a1), b3[xi + second]));
+        const Fq u = !real ? Fq::zero() : g.c ? dbl_raw(a0) : Fq::add_raw(a0, a1);
+        const Fq v = g.c ? a1 : Fq::sub(a0, a1);
+        acc = Fq::wide_add(acc, Fq::mul_wide(u, v));
     }
-    // m = index of the A whose square lane k needs; real part S, t part P
-    const int m = k == 0 || k == 3 ? 0 : (k == 2 || k == 5 ? 1 : 2);
-    const Fq2 sq_a = m == 0 ? sa[0] : (m == 1 ? sa[1] : sa[2]);
-    const Fq2 sq_b = m == 0 ? sb[0] : (m == 1 ? sb[1] : sb[2]);
-    const Fq2 sq_ab = m == 0 ? sab[0] : (m == 1 ? sab[1] : sab[2]);
-    const Fq2 sr = Fq2::add(sq_a, mul_xi(sq_b));
-    const Fq2 pt = Fq2::sub(Fq2::sub(sq_ab, sq_a), sq_b);
-    // k = 0: 3 S0 - 2 f0; 3: 3 P0 + 2 f3; 2: 3 S1 - 2 f2; 5: 3 P1 + 2 f5; 4: 3 S2 - 2 f4; 1: 3 xi P2 + 2 f1
-    const Fq2 term = k == 0 || k == 2 || k == 4 ? sr : (k == 1 ? mul_xi(pt) : pt);
-    const Fq2 t3 = Fq2::add(Fq2::dbl(term), term), f2 = Fq2::dbl(f);
-    return k == 0 || k == 2 || k == 4 ? Fq2::sub(t3, f2) : Fq2::add(t3, f2);
-}
-// f (l0 + l1 w + l3 w^3).
-__device__ __noinline__ Fq2 g_mul_line(const Fq2& f, const Fq2& l0, const Fq2& l1, const Fq2& l3, int k, int base) {
-    const Fq2 x[3] = {f, shfl2(f, base + mod6(k - 1)), shfl2(f, base + mod6(k - 3))};
-    const Fq2 y[3] = {l0, l1, l3};
-    Fq2 p[3];
+    acc = whole_sum<H>(acc);
+    acc = Fq::wide_add(acc, Fq::wide_add(acc, acc));
+    const Fq l = dbl_raw(real ? neg_raw(f) : f);  // -+2 f, times 2^256
+    Fq hi;
 #pragma unroll
-    for (int i = 0; i < 3; ++i) p[i] = Fq2::mul(x[i], y[i]);
-    return Fq2::add(Fq2::add(p[0], k < 1 ? mul_xi(p[1]) : p[1]), k < 3 ? mul_xi(p[2]) : p[2]);
+    for (int w = 0; w < 8; ++w) hi.v[w] = acc.v[8 + w];
+    hi = Fq::add_raw(hi, l);
+#pragma unroll
+    for (int w = 0; w < 8; ++w) acc.v[8 + w] = hi.v[w];
+    return redc_large(acc);
 }
 // f^(q^6): w -> -w.
-DV_INL Fq2 g_conj(const Fq2& f, int k) { return (k & 1) ? Fq2::neg(f) : f; }
-// q^e-power Frobenius, e = 1, 2, 3.
-DV_INL Fq2 g_frob(const Fq2& f, int k, int e) {
-    if (e == 2) return Fq2::mul_fq(f, frob2(k));
-    Fq2 g = frob1(k);
-    if (e == 3) g = Fq2::mul_fq(g, frob2(k));
-    return Fq2::mul(Fq2::conj(f), g);
+DV_INL Fq g_conj(const Fq& f, int k) { return (k & 1) ? Fq::neg(f) : f; }
+// q^e-power Frobenius, e = 1, 2, 3: conj(f_k) xi^(k (q^e - 1) / 6) (f_k itself for e = 2).
+DV_INL Fq g_frob(const Lane& g, const Fq& f, int e) {
+    if (e == 2) return Fq::mul(f, frob2(g.k));
+    Fq2 s = frob1(g.k);
+    if (e == 3) s = Fq2::mul_fq(s, frob2(g.k));
+    const Fq o = shfl_xor_fq(f, 1);
+    // component 0: f0 s0 + f1 s1; component 1: f0 s1 - f1 s0
+    return Fq::mul_sub(o, s.c1, f, g.c ? s.c0 : Fq::neg(s.c0));
 }
-// f^-1 = conj(f) / N, N = f conj(f) in Fq6 (the even lanes, v = w^2).
-__device__ __noinline__ Fq2 g_inv(const Fq2& f, int k, int base) {
-    const Fq2 c = g_conj(f, k);
-    const Fq2 n = g_mul(f, c, k, base);
-    const Fq6 nn = {shfl2(n, base), shfl2(n, base + 2), shfl2(n, base + 4)};
-    const Fq6 ni = f6_inv(nn);
-    const Fq2 mine = (k & 1) ? Fq2::zero() : (k == 0 ? ni.c0 : (k == 2 ? ni.c1 : ni.c2));
-    return g_mul(c, mine, k, base);
+// f^-1 = conj(f) / N, N = f conj(f) in Fq6 (the even coefficients, v = w^2).
+template <int H>
+__device__ __noinline__ Fq g_inv(Fq f, Lane g) {
+    const Fq c = g_conj(f, g.k);
+    const Fq n = g_mul<H>(g, f, c);
+    __syncwarp();
+    if (g.writes) *sm(g.at + SM_V + 2 * g.k + g.c) = n;
+    __syncwarp();
+    const Fq* v = sm(g.at + SM_V);
+    const Fq6 ni = f6_inv({{v[0], v[1]}, {v[4], v[5]}, {v[8], v[9]}});
+    const Fq2 t = g.k == 0 ? ni.c0 : (g.k == 2 ? ni.c1 : ni.c2);
+    return g_mul<H>(g, c, (g.k & 1) ? Fq::zero() : g.c ? t.c1 : t.c0);
 }
 // a^z for a in the cyclotomic subgroup (a^-1 = conj a), z the BN seed, over
 // its width-4 NAF: a, a^3, a^5, a^7 first (one square, three products), then
-// 62 squares and 13 products.
-__device__ __noinline__ Fq2 g_pow_z(const Fq2& a, int k, int base) {
-    Fq2 tab[4];
+// 62 squares and 13 products.  xi times each table entry is kept beside it.
+template <int H>
+__device__ __noinline__ Fq g_pow_z(Fq a, Lane g) {
+    Fq tab[4], xtab[4];
     tab[0] = a;
-    const Fq2 a2 = g_cyc_sqr(a, k, base);
+    const Fq a2 = g_cyc_sqr<H>(a, g), xa2 = xi_part(a2, g.c);
+    xtab[0] = xi_part(a, g.c);
 #pragma unroll 1
-    for (int j = 1; j < 4; ++j) tab[j] = g_mul(tab[j - 1], a2, k, base);
-    Fq2 r = tab[WNAF_Z[0] >> 1];
+    for (int j = 1; j < 4; ++j) {
+        tab[j] = g_mul_staged<H>(g, tab[j - 1], a2, xa2);
+        xtab[j] = xi_part(tab[j], g.c);
+    }
+    Fq r = tab[WNAF_Z[0] >> 1];
 #pragma unroll 1
     for (int i = 1; i < WNAF_Z_LEN; ++i) {
-        r = g_cyc_sqr(r, k, base);
+        r = g_cyc_sqr<H>(r, g);
         const int d = WNAF_Z[i];
         if (d) {
-            const Fq2 t = tab[(d < 0 ? -d : d) >> 1];
-            r = g_mul(r, d > 0 ? t : g_conj(t, k), k, base);
+            const int e = (d < 0 ? -d : d) >> 1;
+            const Fq t = tab[e], x = xtab[e];
+            const bool flip = d < 0 && (g.k & 1);
+            r = g_mul_staged<H>(g, r, flip ? Fq::neg(t) : t, flip ? Fq::neg(x) : x);
         }
     }
     return r;
 }
-DV_INL Fq2 g_one(int k) { return k == 0 ? Fq2::one() : Fq2::zero(); }
+DV_INL Fq g_one(const Lane& g) { return g.k == 0 && g.c == 0 ? Fq::one() : Fq::zero(); }
 
 struct Tw {
-    Fq2 x, y, z;  // Jacobian on the twist
+    Fq x, y, z;  // this lane's components of a Jacobian point on the twist
 };
-
-DV_INL Fq2 pick(int k, const Fq2& v0, const Fq2& v1, const Fq2& v2, const Fq2& v3, const Fq2& v4, const Fq2& v5) {
+DV_INL Fq pick(int k, const Fq& v0, const Fq& v1, const Fq& v2, const Fq& v3, const Fq& v4, const Fq& v5) {
     return k == 0 ? v0 : k == 1 ? v1 : k == 2 ? v2 : k == 3 ? v3 : k == 4 ? v4 : v5;
 }
-// Each lane of the group computes one Fq2 product, its operands chosen by
-// k, and gets every lane's product back.
-DV_INL void level(const Fq2& a, const Fq2& b, int base, Fq2* out, int n) {
-    const Fq2 p = Fq2::mul(a, b);
-#pragma unroll
-    for (int j = 0; j < 6; ++j)
-        if (j < n) out[j] = shfl2(p, base + j);
+// Up to six Fq2 products of a dependency level, product k on the lanes of
+// coefficient k; level_get reads this lane's component of product j.
+template <int H>
+__device__ __noinline__ void level(Fq a, Fq b, Lane g) {
+    __syncwarp();
+    if (g.writes) {
+        *sm(g.at + SM_A + 2 * g.k + g.c) = a;
+        Fq* s = sm(g.at + SM_B + 6 * g.k);
+        s[g.c] = b;
+        if (g.c) s[2] = neg_raw(b);
+    }
+    __syncwarp();
+    Fq::Wide acc = wide_zero();
+    term<H>(acc, g, sm(g.at + SM_A + 2 * g.k), sm(g.at + SM_B + 6 * g.k), 0);
+    const Fq r = Fq::redc(whole_sum<H>(acc));
+    if (g.writes) *sm(g.at + SM_V + 2 * g.k + g.c) = r;
+    __syncwarp();
 }
-DV_INL Fq2 fq2_of(const Fq& x) { return {x, Fq::zero()}; }
+DV_INL Fq level_get(const Lane& g, int j) { return *sm(g.at + SM_V + 2 * j + g.c); }
 
-// T <- 2T and the line's (w^0, w^1, w^3) terms at P, the products spread
-// over the group in three dependency levels:
-//   A = X^2, B = Y^2, ZZ = Z^2, YZ = Y Z;
-//   C = B^2, S = (X + B)^2, E ZZ, Z3 ZZ, E X, E^2   (E = 3A, Z3 = 2 Y Z);
-//   E (D - X3), Z3 ZZ yp, E ZZ xp                   (D = 2(S - A - C), X3 = E^2 - 2D).
-__device__ __noinline__ void dbl_step(Tw& t, const Fq& xp, const Fq& yp, Fq2& l0, Fq2& l1, Fq2& l3, int k, int base) {
-    Fq2 v[6];
-    level(pick(k, t.x, t.y, t.z, t.y, t.x, t.x), pick(k, t.x, t.y, t.z, t.z, t.x, t.x), base, v, 4);
-    const Fq2 a = v[0], b = v[1], zz = v[2];
-    const Fq2 e = Fq2::add(Fq2::dbl(a), a), z3 = Fq2::dbl(v[3]), xb = Fq2::add(t.x, b);
-    level(pick(k, b, xb, e, z3, e, e), pick(k, b, xb, zz, zz, t.x, e), base, v, 6);
-    const Fq2 c = v[0], ezz = v[2], z3zz = v[3], ex = v[4];
-    const Fq2 d = Fq2::dbl(Fq2::sub(Fq2::sub(v[1], a), c));
-    const Fq2 x3 = Fq2::sub(v[5], Fq2::dbl(d));
-    level(pick(k, e, z3zz, ezz, e, e, e), pick(k, Fq2::sub(d, x3), fq2_of(yp), fq2_of(xp), e, e, e), base, v, 3);
-    l0 = v[1];
-    l1 = Fq2::neg(v[2]);
-    l3 = Fq2::sub(ex, Fq2::dbl(b));
-    t.y = Fq2::sub(v[0], Fq2::dbl(Fq2::dbl(Fq2::dbl(c))));
-    t.x = x3;
-    t.z = z3;
-}
-// T <- T + S (S affine) and the line at P, in five levels:
-//   ZZ = Z^2 (every lane); U2 = xs ZZ, ZZZ = Z ZZ;
-//   S2 = ys ZZZ, HH = H^2, (Z + H)^2              (H = U2 - X);
-//   J = H I, V = X I, r^2, r xs, r xp, Z3 ys      (I = 4 HH, r = 2(S2 - Y), Z3 = (Z + H)^2 - ZZ - HH);
-//   r (V - X3), Y J, Z3 yp                        (X3 = r^2 - J - 2V).
-__device__ __noinline__ void add_step(Tw& t, const Fq2& xs, const Fq2& ys, const Fq& xp, const Fq& yp, Fq2& l0,
-                                      Fq2& l1, Fq2& l3, int k, int base) {
-    Fq2 v[6];
-    const Fq2 zz = Fq2::mul(t.z, t.z);
-    level(pick(k, xs, t.z, xs, xs, xs, xs), pick(k, zz, zz, zz, zz, zz, zz), base, v, 2);
-    const Fq2 h = Fq2::sub(v[0], t.x), zh = Fq2::add(t.z, h);
-    level(pick(k, ys, h, zh, h, h, h), pick(k, v[1], h, zh, h, h, h), base, v, 3);
-    const Fq2 hh = v[1];
-    const Fq2 i = Fq2::dbl(Fq2::dbl(hh));
-    const Fq2 r = Fq2::dbl(Fq2::sub(v[0], t.y));
-    const Fq2 z3 = Fq2::sub(Fq2::sub(v[2], zz), hh);
-    level(pick(k, h, t.x, r, r, r, z3), pick(k, i, i, r, xs, fq2_of(xp), ys), base, v, 6);
-    const Fq2 j = v[0], vv = v[1], rxs = v[3], rxp = v[4], z3ys = v[5];
-    const Fq2 x3 = Fq2::sub(Fq2::sub(v[2], j), Fq2::dbl(vv));
-    level(pick(k, r, t.y, z3, r, r, r), pick(k, Fq2::sub(vv, x3), j, fq2_of(yp), r, r, r), base, v, 3);
-    l0 = v[2];
-    l1 = Fq2::neg(rxp);
-    l3 = Fq2::sub(rxs, z3ys);
-    t.y = Fq2::sub(v[0], Fq2::dbl(v[1]));
-    t.x = x3;
-    t.z = z3;
-}
-
-struct GroupLane {
-    int k, base;
-    uint64_t group;  // global group index
-    bool live;       // lanes 0..29 of the warp
-};
-DV_INL GroupLane group_lane() {
-    const int l = threadIdx.x & 31;
-    const int k = l < GL * GROUPS_PER_WARP ? l % GL : l - GL * GROUPS_PER_WARP;
-    const uint64_t warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    return {k, l - k, warp * GROUPS_PER_WARP + (uint64_t)(l / GL), l < GL * GROUPS_PER_WARP};
-}
-
-// ------------------------------------------------------------------ prepared G2 points
 // A line of the Miller loop at P = (xp, yp) is A yp + (B xp) w + C w^3 with
 // A, B, C depending on Q alone (the doubling: A = 2 Y Z^3, B = -3 X^2 Z^2,
 // C = 3 X^3 - 2 Y^2; the addition: A = 2 Z H, B = -2 R, C = 2 R xs - 2 Z H ys).
@@ -387,140 +471,116 @@ DV_INL GroupLane group_lane() {
 struct __align__(16) Line {
     Fq2 a, b, c;
 };
+struct LinePart {
+    Fq a, b, c;  // this lane's components
+};
 constexpr int LINES = 88;  // 65 doublings, 21 NAF additions (nonzero digits after the first), 2 Frobenius additions
 
-// The doubling and addition steps without P: the same levels, minus the
-// products by xp and yp.
-__device__ __noinline__ void prep_dbl(Tw& t, Line& l, int k, int base) {
-    Fq2 v[6];
-    level(pick(k, t.x, t.y, t.z, t.y, t.x, t.x), pick(k, t.x, t.y, t.z, t.z, t.x, t.x), base, v, 4);
-    const Fq2 a = v[0], b = v[1], zz = v[2];
-    const Fq2 e = Fq2::add(Fq2::dbl(a), a), z3 = Fq2::dbl(v[3]), xb = Fq2::add(t.x, b);
-    level(pick(k, b, xb, e, z3, e, e), pick(k, b, xb, zz, zz, t.x, e), base, v, 6);
-    const Fq2 c = v[0], ezz = v[2], z3zz = v[3], ex = v[4];
-    const Fq2 d = Fq2::dbl(Fq2::sub(Fq2::sub(v[1], a), c));
-    const Fq2 x3 = Fq2::sub(v[5], Fq2::dbl(d));
-    level(e, Fq2::sub(d, x3), base, v, 1);
-    l = {z3zz, Fq2::neg(ezz), Fq2::sub(ex, Fq2::dbl(b))};
-    t.y = Fq2::sub(v[0], Fq2::dbl(Fq2::dbl(Fq2::dbl(c))));
+// T <- 2T and its line, the products in three levels:
+//   A = X^2, B = Y^2, ZZ = Z^2, YZ = Y Z;
+//   C = B^2, (X + B)^2, E ZZ, Z3 ZZ, E X, E^2   (E = 3A, Z3 = 2 Y Z);
+//   E (D - X3)                                  (D = 2((X + B)^2 - A - C), X3 = E^2 - 2D).
+template <int H>
+__device__ __noinline__ LinePart prep_dbl(Tw& t, Lane g) {
+    level<H>(pick(g.k, t.x, t.y, t.z, t.y, t.x, t.x), pick(g.k, t.x, t.y, t.z, t.z, t.x, t.x), g);
+    const Fq a = level_get(g, 0), b = level_get(g, 1), zz = level_get(g, 2);
+    const Fq e = Fq::add(Fq::dbl(a), a), z3 = Fq::dbl(level_get(g, 3)), xb = Fq::add(t.x, b);
+    level<H>(pick(g.k, b, xb, e, z3, e, e), pick(g.k, b, xb, zz, zz, t.x, e), g);
+    const Fq c = level_get(g, 0), ezz = level_get(g, 2), z3zz = level_get(g, 3), ex = level_get(g, 4);
+    const Fq d = Fq::dbl(Fq::sub(Fq::sub(level_get(g, 1), a), c));
+    const Fq x3 = Fq::sub(level_get(g, 5), Fq::dbl(d));
+    level<H>(e, Fq::sub(d, x3), g);
+    t.y = Fq::sub(level_get(g, 0), Fq::dbl(Fq::dbl(Fq::dbl(c))));
     t.x = x3;
     t.z = z3;
+    return {z3zz, Fq::neg(ezz), Fq::sub(ex, Fq::dbl(b))};
 }
-__device__ __noinline__ void prep_add(Tw& t, const Fq2& xs, const Fq2& ys, Line& l, int k, int base) {
-    Fq2 v[6];
-    const Fq2 zz = Fq2::mul(t.z, t.z);
-    level(pick(k, xs, t.z, xs, xs, xs, xs), pick(k, zz, zz, zz, zz, zz, zz), base, v, 2);
-    const Fq2 h = Fq2::sub(v[0], t.x), zh = Fq2::add(t.z, h);
-    level(pick(k, ys, h, zh, h, h, h), pick(k, v[1], h, zh, h, h, h), base, v, 3);
-    const Fq2 hh = v[1];
-    const Fq2 i = Fq2::dbl(Fq2::dbl(hh));
-    const Fq2 r = Fq2::dbl(Fq2::sub(v[0], t.y));
-    const Fq2 z3 = Fq2::sub(Fq2::sub(v[2], zz), hh);
-    level(pick(k, h, t.x, r, r, z3, r), pick(k, i, i, r, xs, ys, r), base, v, 5);
-    const Fq2 j = v[0], vv = v[1], rxs = v[3], z3ys = v[4];
-    const Fq2 x3 = Fq2::sub(Fq2::sub(v[2], j), Fq2::dbl(vv));
-    level(pick(k, r, t.y, r, r, r, r), pick(k, Fq2::sub(vv, x3), j, r, r, r, r), base, v, 2);
-    l = {z3, Fq2::neg(r), Fq2::sub(rxs, z3ys)};
-    t.y = Fq2::sub(v[0], Fq2::dbl(v[1]));
+// T <- T + S (S affine) and its line, in five levels:
+//   ZZ = Z^2; U2 = xs ZZ, ZZZ = Z ZZ;
+//   S2 = ys ZZZ, HH = H^2, (Z + H)^2            (H = U2 - X);
+//   J = H I, V = X I, r^2, r xs, Z3 ys          (I = 4 HH, r = 2(S2 - Y), Z3 = (Z + H)^2 - ZZ - HH);
+//   r (V - X3), Y J                             (X3 = r^2 - J - 2V).
+template <int H>
+__device__ __noinline__ LinePart prep_add(Tw& t, Fq xs, Fq ys, Lane g) {
+    level<H>(t.z, t.z, g);
+    const Fq zz = level_get(g, 0);
+    level<H>(pick(g.k, xs, t.z, xs, xs, xs, xs), zz, g);
+    const Fq h = Fq::sub(level_get(g, 0), t.x), zh = Fq::add(t.z, h), zzz = level_get(g, 1);
+    level<H>(pick(g.k, ys, h, zh, h, h, h), pick(g.k, zzz, h, zh, h, h, h), g);
+    const Fq hh = level_get(g, 1);
+    const Fq i = Fq::dbl(Fq::dbl(hh));
+    const Fq r = Fq::dbl(Fq::sub(level_get(g, 0), t.y));
+    const Fq z3 = Fq::sub(Fq::sub(level_get(g, 2), zz), hh);
+    level<H>(pick(g.k, h, t.x, r, r, z3, r), pick(g.k, i, i, r, xs, ys, r), g);
+    const Fq j = level_get(g, 0), vv = level_get(g, 1), rxs = level_get(g, 3), z3ys = level_get(g, 4);
+    const Fq x3 = Fq::sub(Fq::sub(level_get(g, 2), j), Fq::dbl(vv));
+    level<H>(pick(g.k, r, t.y, r, r, r, r), pick(g.k, Fq::sub(vv, x3), j, r, r, r, r), g);
+    t.y = Fq::sub(level_get(g, 0), Fq::dbl(level_get(g, 1)));
     t.x = x3;
     t.z = z3;
+    return {z3, Fq::neg(r), Fq::sub(rxs, z3ys)};
+}
+// The loop over the lines of Q in order: put(line) for each.
+template <int H, class Put>
+DV_INL void for_lines(const G2A& q, const Lane& g, Put&& put) {
+    const Fq qx = g.c ? q.x.c1 : q.x.c0, qy = g.c ? q.y.c1 : q.y.c0, nqy = Fq::neg(qy);
+    Tw t{qx, qy, g.c ? Fq::zero() : Fq::one()};
+#pragma unroll 1
+    for (int i = 1; i < NAF_LEN; ++i) {
+        put(prep_dbl<H>(t, g), i > 1);
+        const int d = NAF_6Z2[i];
+        if (d) put(prep_add<H>(t, qx, d > 0 ? qy : nqy, g), false);
+    }
+    // pi(Q) = (conj(x) xi^((q-1)/3), conj(y) xi^((q-1)/2)); -pi^2(Q) = (x xi^((q^2-1)/3), -y xi^((q^2-1)/2))
+    const Fq2 x1 = Fq2::mul(Fq2::conj(q.x), frob1(2)), y1 = Fq2::mul(Fq2::conj(q.y), frob1(3));
+    put(prep_add<H>(t, g.c ? x1.c1 : x1.c0, g.c ? y1.c1 : y1.c0, g), false);
+    put(prep_add<H>(t, Fq::mul(qx, frob2(2)), Fq::neg(Fq::mul(qy, frob2(3))), g), false);
 }
 
 // The LINES triples of every Q (one lane group each) at lines[LINES q ..],
 // and inf[q] = 1 for Q at infinity (whose lines count as 1).
-__global__ void __launch_bounds__(128) k_prepare(const G2A* __restrict__ g2, uint64_t nq, Line* __restrict__ lines,
-                                                 uint32_t* __restrict__ inf) {
-    const GroupLane g = group_lane();
-    const bool mine = g.live && g.group < nq;
-    const uint64_t qi = mine ? g.group : 0;
+template <int H>
+__global__ void __launch_bounds__(THREADS) k_prepare(const G2A* __restrict__ g2, uint64_t nq, Line* __restrict__ lines,
+                                                     uint32_t* __restrict__ inf) {
+    const Lane g = lane_setup<H>();
+    const bool mine = g.writes && g.group < nq;
+    const uint64_t qi = g.group < nq ? g.group : 0;
     const G2A q = g2[qi];
-    if (mine && g.k == 0) inf[qi] = q.is_inf() ? 1u : 0u;
-    Line* out = lines + (uint64_t)LINES * qi;
-    Tw t{q.x, q.y, Fq2::one()};
-    Line l;
-    int n = 0;
-    const Fq2 nqy = Fq2::neg(q.y);
-    auto put = [&](const Line& x) {
-        if (mine && g.k < 3) (&out[n].a)[g.k] = (&x.a)[g.k];
-        ++n;
-    };
-    for (int i = 1; i < NAF_LEN; ++i) {
-        prep_dbl(t, l, g.k, g.base);
-        put(l);
-        const int d = NAF_6Z2[i];
-        if (d) {
-            prep_add(t, q.x, d > 0 ? q.y : nqy, l, g.k, g.base);
-            put(l);
-        }
-    }
-    const Fq2 x1 = Fq2::mul(Fq2::conj(q.x), frob1(2)), y1 = Fq2::mul(Fq2::conj(q.y), frob1(3));
-    const Fq2 x2 = Fq2::mul_fq(q.x, frob2(2)), y2 = Fq2::neg(Fq2::mul_fq(q.y, frob2(3)));
-    prep_add(t, x1, y1, l, g.k, g.base);
-    put(l);
-    prep_add(t, x2, y2, l, g.k, g.base);
-    put(l);
+    if (mine && g.k == 0 && g.c == 0) inf[qi] = q.is_inf() ? 1u : 0u;
+    Fq* out = reinterpret_cast<Fq*>(lines + (uint64_t)LINES * qi) + 2 * g.k + g.c;
+    for_lines<H>(q, g, [&](const LinePart& l, bool) {
+        if (mine && g.k < 3) *out = g.k == 0 ? l.a : g.k == 1 ? l.b : l.c;
+        out += sizeof(Line) / sizeof(Fq);
+    });
 }
 
-// A line A yp + (B xp) w + C w^3 scaled to its P: coefficients of w^0,
-// w^1, w^3.  A term with P or Q at infinity, or past its equation's count,
-// takes the line 1.
-struct SLine {
-    Fq2 l0, l1, l3;
-};
-DV_INL SLine line_one() { return {Fq2::one(), Fq2::zero(), Fq2::zero()}; }
-// One term's scaling: the four base products A yp, B xp one per lane
-// (lanes 0..3), shared by shuffles.
-DV_INL SLine scale_one(const Line& x, const G1A& p, bool one, int k, int base) {
-    const Fq u = k == 0 ? x.a.c0 : k == 1 ? x.a.c1 : k == 2 ? x.b.c0 : x.b.c1;
-    const Fq r = Fq::mul(u, k < 2 ? p.y : p.x);
-    const SLine l = {{shfl_fq(r, base), shfl_fq(r, base + 1)}, {shfl_fq(r, base + 2), shfl_fq(r, base + 3)}, x.c};
-    return one ? line_one() : l;
-}
-// Two terms' scaling: eight base products, lane k forms product k and lanes
-// 0, 1 also products 6, 7 (x: A yp, B xp of the first term, then of the
-// second).
-DV_INL void scale_two(const Line& x, const G1A& p, bool one_x, const Line& y, const G1A& q, bool one_y, int k,
-                      int base, SLine& a, SLine& b) {
-    const Fq u0 = k == 0 ? x.a.c0 : k == 1 ? x.a.c1 : k == 2 ? x.b.c0 : k == 3 ? x.b.c1 : k == 4 ? y.a.c0 : y.a.c1;
-    const Fq v0 = k < 2 ? p.y : (k < 4 ? p.x : q.y);
-    const Fq::Pair r = Fq::mul2(u0, v0, k == 0 ? y.b.c0 : y.b.c1, q.x);
-    const SLine la = {{shfl_fq(r.r0, base), shfl_fq(r.r0, base + 1)}, {shfl_fq(r.r0, base + 2), shfl_fq(r.r0, base + 3)},
-                      x.c};
-    const SLine lb = {{shfl_fq(r.r0, base + 4), shfl_fq(r.r0, base + 5)}, {shfl_fq(r.r1, base), shfl_fq(r.r1, base + 1)},
-                      y.c};
-    a = one_x ? line_one() : la;
-    b = one_y ? line_one() : lb;
-}
-// (a0 + a1 w + a3 w^3)(b0 + b1 w + b3 w^3): the Karatsuba products p0 = a0 b0,
-// p1 = a1 b1, p2 = a3 b3, p3 = (a0 + a1)(b0 + b1), p4 = (a0 + a3)(b0 + b3),
-// p5 = (a1 + a3)(b1 + b3), one per lane; c0 = p0 + xi p2, c1 = p3 - p0 - p1,
-// c2 = p1, c3 = p4 - p0 - p2, c4 = p5 - p1 - p2, c5 = 0.
-__device__ __noinline__ Fq2 g_line_line(const SLine& a, const SLine& b, int k, int base) {
-    const Fq2 x = k == 0 ? a.l0 : k == 1 ? a.l1 : k == 2 ? a.l3 : Fq2::add(k == 5 ? a.l1 : a.l0, k == 3 ? a.l1 : a.l3);
-    const Fq2 y = k == 0 ? b.l0 : k == 1 ? b.l1 : k == 2 ? b.l3 : Fq2::add(k == 5 ? b.l1 : b.l0, k == 3 ? b.l1 : b.l3);
-    const Fq2 p = Fq2::mul(x, y);
-    const Fq2 m = shfl2(p, base + (k == 1 ? 3 : k == 2 ? 1 : k == 3 ? 4 : k == 4 ? 5 : 0));
-    const Fq2 p0 = shfl2(p, base), p1 = shfl2(p, base + 1), p2 = shfl2(p, base + 2);
-    const Fq2 d = Fq2::sub(Fq2::sub(m, k == 4 ? p1 : p0), k == 1 ? p1 : p2);
-    return k == 0 ? Fq2::add(p0, mul_xi(p2)) : k == 2 ? m : k == 5 ? Fq2::zero() : d;
+// This lane's component of a line scaled to P (on lanes k = 0, 1, 3): raw is
+// its component of A, B or C; one: the line counts as 1.
+DV_INL Fq scaled_line(const Lane& g, const Fq& raw, const Fq& coord, bool one) {
+    const Fq s = Fq::mul(raw, coord);
+    const Fq v = g.k == 3 ? raw : s;
+    return one ? g_one(g) : v;
 }
 
 // Miller value of every equation from its terms' P and prepared Q, one lane
 // group per equation and one f for all its terms (the multi-Miller loop):
-// every step squares f once and multiplies in the lines of all the terms,
-// two terms' lines first multiplied together (six Fq2 products, one per
-// lane) and then into f by one product, a last odd term by the sparse line
-// product.  Every group of a warp runs the warp's largest term count.
-// Value of equation e at out[6 e + k]; without offsets every term is its own
-// equation (a group per term, for batches too small to fill the GPU, whose
-// terms then meet in the final exponentiation).
-__global__ void __launch_bounds__(128) k_miller_multi(const G1A* __restrict__ g1, const uint32_t* __restrict__ qidx,
-                                                      const uint32_t* __restrict__ qinf,
-                                                      const Line* __restrict__ lines,
-                                                      const uint64_t* __restrict__ offsets, uint64_t equations,
-                                                      Fq2* __restrict__ out) {
-    const GroupLane g = group_lane();
-    const bool mine = g.live && g.group < equations;
+// every step squares f once and multiplies in the lines of all the terms.
+// Every group of a warp runs the warp's largest term count.  The next line
+// and coordinate are loaded before the current product.  Component c of
+// coefficient k of equation e at out[12 e + 2 k + c]; without offsets every
+// term is its own equation (a group per term, for batches too small to fill
+// the GPU, whose terms then meet in the final exponentiation).
+// Measured (the terms of one proof's 49 equations): 909 us with six lanes a
+// group and Karatsuba products, 343 us with H = 2.
+template <int H>
+__global__ void __launch_bounds__(THREADS) k_miller_multi(const G1A* __restrict__ g1,
+                                                          const uint32_t* __restrict__ qidx,
+                                                          const uint32_t* __restrict__ qinf,
+                                                          const Line* __restrict__ lines,
+                                                          const uint64_t* __restrict__ offsets, uint64_t equations,
+                                                          Fq* __restrict__ out) {
+    const Lane g = lane_setup<H>();
+    const bool mine = g.group < equations;
     const uint64_t e = mine ? g.group : 0;
     const uint64_t first = !mine ? 0 : offsets ? offsets[e] : e;
     const uint64_t count = !mine ? 0 : offsets ? offsets[e + 1] - first : 1;
@@ -531,111 +591,99 @@ __global__ void __launch_bounds__(128) k_miller_multi(const G1A* __restrict__ g1
         most = o > most ? o : most;
     }
     // term j of this group at line n (term 0 of the call stands in past the
-    // group's count, which is then nonzero somewhere in the warp); true when
-    // its line counts as 1
-    auto term = [&](uint64_t j, int n, G1A& p, Line& l) {
+    // group's count, which is then nonzero somewhere in the warp)
+    const int part = 2 * (g.k == 1 ? 1 : g.k == 3 ? 2 : 0) + g.c;
+    auto fetch = [&](uint64_t j, int n, Fq& raw, Fq& coord, bool& one) {
         const bool have = j < count;
         const uint64_t t = have ? first + j : 0;
-        p = g1[t];
+        const G1A p = g1[t];
         const uint32_t qi = qidx[t];
-        l = lines[(uint64_t)LINES * qi + n];
-        return !have || p.is_inf() || qinf[qi] != 0;
+        raw = reinterpret_cast<const Fq*>(lines + (uint64_t)LINES * qi + n)[part];
+        coord = g.k == 1 ? p.x : p.y;
+        one = !have || p.is_inf() || qinf[qi] != 0;
     };
-    Fq2 f = g_one(g.k);
-    auto apply = [&](int n) {
-        for (uint64_t j = 0; j < most; j += 2) {
-            G1A pa, pb;
-            Line la, lb;
-            const bool oa = term(j, n, pa, la);
-            if (j + 1 < most) {
-                const bool ob = term(j + 1, n, pb, lb);
-                SLine a, b;
-                scale_two(la, pa, oa, lb, pb, ob, g.k, g.base, a, b);
-                f = g_mul(f, g_line_line(a, b, g.k, g.base), g.k, g.base);
+    Fq f = g_one(g);
+    if (most) {
+        Fq raw, coord;
+        bool one;
+        fetch(0, 0, raw, coord, one);
+        int n = 0, extra = 0;  // extra: the step's second line (an addition) comes next
+#pragma unroll 1
+        for (int i = 1; n < LINES;) {
+            if (i > 1 && i < NAF_LEN && !extra) f = g_sqr<H>(g, f);
+#pragma unroll 1
+            for (uint64_t j = 0; j < most; ++j) {
+                const Fq r = raw, c = coord;
+                const bool o = one;
+                const bool last = j + 1 == most;
+                if (!last || n + 1 < LINES) fetch(last ? 0 : j + 1, last ? n + 1 : n, raw, coord, one);
+                f = g_mul_line<H>(g, f, scaled_line(g, r, c, o));
+            }
+            ++n;
+            if (i < NAF_LEN && !extra && NAF_6Z2[i]) {
+                extra = 1;
             } else {
-                const SLine a = scale_one(la, pa, oa, g.k, g.base);
-                f = g_mul_line(f, a.l0, a.l1, a.l3, g.k, g.base);
+                extra = 0;
+                ++i;
             }
         }
-    };
-    int n = 0;
-    for (int i = 1; i < NAF_LEN; ++i) {
-        if (i > 1) f = g_sqr(f, g.k, g.base);
-        apply(n++);
-        if (NAF_6Z2[i]) apply(n++);
     }
-    apply(n++);
-    apply(n++);
-    if (mine) out[6 * e + g.k] = f;
+    if (mine && g.writes) out[12 * e + 2 * g.k + g.c] = f;
 }
 
-// Miller value of (P, Q) as this lane's coefficient; every lane holds T and
-// the lines (their products are spread over the group).
-__device__ Fq2 g_miller(const G1A& p, const G2A& q, int k, int base) {
-    Tw t{q.x, q.y, Fq2::one()};
-    Fq2 f = g_one(k);
-    Fq2 l0, l1, l3;
-    const Fq2 nqy = Fq2::neg(q.y);
-    for (int i = 1; i < NAF_LEN; ++i) {
-        dbl_step(t, p.x, p.y, l0, l1, l3, k, base);
-        f = g_mul_line(g_sqr(f, k, base), l0, l1, l3, k, base);
-        const int d = NAF_6Z2[i];
-        if (d) {
-            add_step(t, q.x, d > 0 ? q.y : nqy, p.x, p.y, l0, l1, l3, k, base);
-            f = g_mul_line(f, l0, l1, l3, k, base);
-        }
-    }
-    // pi(Q) = (conj(x) xi^((q-1)/3), conj(y) xi^((q-1)/2)); -pi^2(Q) = (x xi^((q^2-1)/3), -y xi^((q^2-1)/2))
-    const Fq2 x1 = Fq2::mul(Fq2::conj(q.x), frob1(2)), y1 = Fq2::mul(Fq2::conj(q.y), frob1(3));
-    const Fq2 x2 = Fq2::mul_fq(q.x, frob2(2)), y2 = Fq2::neg(Fq2::mul_fq(q.y, frob2(3)));
-    add_step(t, x1, y1, p.x, p.y, l0, l1, l3, k, base);
-    f = g_mul_line(f, l0, l1, l3, k, base);
-    add_step(t, x2, y2, p.x, p.y, l0, l1, l3, k, base);
-    return g_mul_line(f, l0, l1, l3, k, base);
+template <int H>
+__device__ Fq g_final_exponentiation(Fq m, const Lane& g) {
+    const auto mul = [&](const Fq& a, const Fq& b) { return g_mul<H>(g, a, b); };
+    const auto sqr = [&](const Fq& a) { return g_cyc_sqr<H>(a, g); };
+    Fq f = mul(g_conj(m, g.k), g_inv<H>(m, g));  // ^(q^6 - 1)
+    f = mul(g_frob(g, f, 2), f);                  // ^(q^2 + 1)
+    const Fq a = g_pow_z<H>(f, g);
+    const Fq b = g_pow_z<H>(a, g);
+    const Fq c = g_pow_z<H>(b, g);
+    const Fq a2 = sqr(a), a4 = sqr(a2), a6 = mul(a4, a2);
+    const Fq b2 = sqr(b), b6 = mul(sqr(b2), b2);
+    const Fq b12 = sqr(b6);
+    const Fq c4 = sqr(sqr(c)), c12 = mul(sqr(c4), c4);
+    const Fq tt = mul(c12, b6);
+    const Fq l1 = mul(tt, a4);
+    const Fq l2 = mul(tt, a6);
+    const Fq l3 = mul(l1, g_conj(f, g.k));
+    const Fq l0 = mul(mul(mul(c12, b12), a6), f);
+    Fq r = mul(l0, g_frob(g, l1, 1));
+    r = mul(r, g_frob(g, l2, 2));
+    return mul(r, g_frob(g, l3, 3));
 }
 
-__device__ Fq2 g_final_exponentiation(const Fq2& m, int k, int base) {
-    Fq2 f = g_mul(g_conj(m, k), g_inv(m, k, base), k, base);  // ^(q^6 - 1)
-    f = g_mul(g_frob(f, k, 2), f, k, base);                    // ^(q^2 + 1)
-    const Fq2 a = g_pow_z(f, k, base);
-    const Fq2 b = g_pow_z(a, k, base);
-    const Fq2 c = g_pow_z(b, k, base);
-    const Fq2 a2 = g_cyc_sqr(a, k, base), a4 = g_cyc_sqr(a2, k, base), a6 = g_mul(a4, a2, k, base);
-    const Fq2 b2 = g_cyc_sqr(b, k, base), b6 = g_mul(g_cyc_sqr(b2, k, base), b2, k, base);
-    const Fq2 b12 = g_cyc_sqr(b6, k, base);
-    const Fq2 c4 = g_cyc_sqr(g_cyc_sqr(c, k, base), k, base), c12 = g_mul(g_cyc_sqr(c4, k, base), c4, k, base);
-    const Fq2 tt = g_mul(c12, b6, k, base);
-    const Fq2 l1 = g_mul(tt, a4, k, base);
-    const Fq2 l2 = g_mul(tt, a6, k, base);
-    const Fq2 l3 = g_mul(l1, g_conj(f, k), k, base);
-    const Fq2 l0 = g_mul(g_mul(g_mul(c12, b12, k, base), a6, k, base), f, k, base);
-    Fq2 r = g_mul(l0, g_frob(l1, k, 1), k, base);
-    r = g_mul(r, g_frob(l2, k, 2), k, base);
-    return g_mul(r, g_frob(l3, k, 3), k, base);
-}
-
-// Miller value of every term, one lane group per term (coefficient k of
-// term t at out[6 t + k]); infinity on either side gives one.
-__global__ void __launch_bounds__(128) k_miller(const G1A* __restrict__ g1, const G2A* __restrict__ g2,
-                                                uint64_t terms, Fq2* __restrict__ out) {
-    const GroupLane g = group_lane();
-    const bool mine = g.live && g.group < terms;
-    const uint64_t t = mine ? g.group : 0;  // idle lanes compute on term 0
+// Miller value of every term, one lane group per term (layout as above),
+// for G2 points that do not repeat; infinity on either side gives one.
+template <int H>
+__global__ void __launch_bounds__(THREADS) k_miller(const G1A* __restrict__ g1, const G2A* __restrict__ g2,
+                                                    uint64_t terms, Fq* __restrict__ out) {
+    const Lane g = lane_setup<H>();
+    const bool mine = g.group < terms;
+    const uint64_t t = mine ? g.group : 0;  // idle groups compute on term 0
     const G1A p = g1[t];
     const G2A q = g2[t];
-    const Fq2 f = g_miller(p, q, g.k, g.base);
-    if (mine) out[6 * t + g.k] = (p.is_inf() || q.is_inf()) ? g_one(g.k) : f;
+    const Fq coord = g.k == 1 ? p.x : p.y;
+    Fq f = g_one(g);
+    for_lines<H>(q, g, [&](const LinePart& l, bool square) {
+        if (square) f = g_sqr<H>(g, f);
+        f = g_mul_line<H>(g, f, scaled_line(g, g.k == 0 ? l.a : g.k == 1 ? l.b : l.c, coord, false));
+    });
+    if (mine && g.writes) out[12 * t + 2 * g.k + g.c] = (p.is_inf() || q.is_inf()) ? g_one(g) : f;
 }
 
 // One lane group per equation: product of its terms' values (every group of
 // a warp runs the warp's largest term count, multiplying by one past its
 // own; without offsets one value per equation), final exponentiation,
 // verdict, and with gt the canonical GT element.
-__global__ void __launch_bounds__(128) k_final_exp(const Fq2* __restrict__ miller, const uint64_t* __restrict__ offsets,
-                                                   uint64_t equations, uint8_t* __restrict__ verdicts,
-                                                   uint8_t* __restrict__ gt) {
-    const GroupLane g = group_lane();
-    const bool mine = g.live && g.group < equations;
+// Measured (49 equations): 1383 us with six lanes a group, 488 us with H = 2.
+template <int H>
+__global__ void __launch_bounds__(THREADS) k_final_exp(const Fq* __restrict__ miller,
+                                                       const uint64_t* __restrict__ offsets, uint64_t equations,
+                                                       uint8_t* __restrict__ verdicts, uint8_t* __restrict__ gt) {
+    const Lane g = lane_setup<H>();
+    const bool mine = g.group < equations;
     const uint64_t e = mine ? g.group : 0;
     const uint64_t first = !mine ? 0 : offsets ? offsets[e] : e;
     const uint64_t count = !mine ? 0 : offsets ? offsets[e + 1] - first : 1;
@@ -645,39 +693,74 @@ __global__ void __launch_bounds__(128) k_final_exp(const Fq2* __restrict__ mille
         const uint64_t o = __shfl_xor_sync(FULL, most, off);
         most = o > most ? o : most;
     }
-    Fq2 f = g_one(g.k);
+    Fq f = g_one(g);
+#pragma unroll 1
     for (uint64_t t = 0; t < most; ++t) {
-        const Fq2 v = t < count ? miller[6 * (first + t) + g.k] : g_one(g.k);
-        f = t == 0 ? v : g_mul(f, v, g.k, g.base);
+        const Fq v = t < count ? miller[12 * (first + t) + 2 * g.k + g.c] : g_one(g);
+        f = t == 0 ? v : g_mul<H>(g, f, v);
     }
-    const Fq2 r = g_final_exponentiation(f, g.k, g.base);
-    const bool coef_ok = g.k == 0 ? (r.c0 == Fq::one() && r.c1.is_zero()) : r.is_zero();
-    const unsigned ok = __ballot_sync(FULL, coef_ok);
-    if (!mine) return;
-    if (verdicts && g.k == 0) verdicts[e] = ((ok >> g.base) & 0x3fu) == 0x3fu ? 1 : 0;
+    const Fq r = g_final_exponentiation<H>(f, g);
+    const bool ok = g.k == 0 && g.c == 0 ? r == Fq::one() : r.is_zero();
+    const unsigned all = __ballot_sync(FULL, ok) >> (H == 1 ? threadIdx.x & 16 : 0);
+    if (!mine || !g.writes) return;
+    if (verdicts && g.k == 0 && g.c == 0) verdicts[e] = (all & 0xfffu) == 0xfffu ? 1 : 0;
     if (gt) {
         // tower order: w^0, w^2, w^4, w^1, w^3, w^5
         const int slot = (g.k & 1) ? 3 + (g.k >> 1) : (g.k >> 1);
-        store_canonical(gt + 384 * e + 64 * slot, r.c0);
-        store_canonical(gt + 384 * e + 64 * slot + 32, r.c1);
+        store_canonical(gt + 384 * e + 64 * slot + 32 * g.c, r);
     }
 }
 
 constexpr uint64_t PREP_MAX = 1ull << 17;  // distinct G2 points prepared in one call (17.5 KB each)
 
-constexpr uint64_t GROUPS_PER_BLOCK = 128 / 32 * GROUPS_PER_WARP;
-
-unsigned group_blocks(uint64_t groups) { return (unsigned)((groups + GROUPS_PER_BLOCK - 1) / GROUPS_PER_BLOCK); }
+// Whether a call of this many groups gives each the whole warp: while that
+// leaves at most two warps on each SM quarter, where the multiply pipe is
+// busy.  Limits of one, two and four warps measured the same to 1 % on one
+// proof's checks and on 32 proofs'; 4096 equations take 3.78 ms (5.26 ms
+// with six lanes a group), one alone 0.83 ms (2.82 ms).
+constexpr uint64_t SPLIT_WARPS = 2;
+bool split_groups(uint64_t groups) { return groups <= SPLIT_WARPS * 4 * (uint64_t)sm_count(); }
+template <int H>
+unsigned group_blocks(uint64_t groups) {
+    return (unsigned)((groups + GROUPS_PER_BLOCK<H> - 1) / GROUPS_PER_BLOCK<H>);
+}
+void launch_prepare(const G2A* q, uint64_t nq, Line* lines, uint32_t* inf, cudaStream_t st) {
+    if (split_groups(nq)) k_prepare<2><<<group_blocks<2>(nq), THREADS, SM_BYTES<2>, st>>>(q, nq, lines, inf);
+    else k_prepare<1><<<group_blocks<1>(nq), THREADS, SM_BYTES<1>, st>>>(q, nq, lines, inf);
+    DV_LAUNCH();
+}
+void launch_miller(const G1A* p, const G2A* q, uint64_t terms, Fq* out, cudaStream_t st) {
+    if (split_groups(terms)) k_miller<2><<<group_blocks<2>(terms), THREADS, SM_BYTES<2>, st>>>(p, q, terms, out);
+    else k_miller<1><<<group_blocks<1>(terms), THREADS, SM_BYTES<1>, st>>>(p, q, terms, out);
+    DV_LAUNCH();
+}
+// d_off null: one group per term
+void launch_miller_multi(const G1A* p, const uint32_t* qidx, const uint32_t* qinf, const Line* lines,
+                         const uint64_t* d_off, uint64_t groups, Fq* out, cudaStream_t st) {
+    if (split_groups(groups))
+        k_miller_multi<2><<<group_blocks<2>(groups), THREADS, SM_BYTES<2>, st>>>(p, qidx, qinf, lines, d_off, groups, out);
+    else
+        k_miller_multi<1><<<group_blocks<1>(groups), THREADS, SM_BYTES<1>, st>>>(p, qidx, qinf, lines, d_off, groups, out);
+    DV_LAUNCH();
+}
+void launch_final_exp(const Fq* mil, const uint64_t* d_off, uint64_t equations, uint8_t* verdicts, uint8_t* gt,
+                      cudaStream_t st) {
+    if (split_groups(equations))
+        k_final_exp<2><<<group_blocks<2>(equations), THREADS, SM_BYTES<2>, st>>>(mil, d_off, equations, verdicts, gt);
+    else
+        k_final_exp<1><<<group_blocks<1>(equations), THREADS, SM_BYTES<1>, st>>>(mil, d_off, equations, verdicts, gt);
+    DV_LAUNCH();
+}
 
 // Whether the prepared Miller loops run one group per equation (the
-// multi-Miller loop, fewer instructions) rather than one per term (shorter
-// chains): per equation once a group per term would take more than one wave
-// of resident blocks (on B200, 2 blocks of 20 groups per SM: 5920 terms).
+// multi-Miller loop, one square of f for all terms) rather than one per term
+// (shorter chains): per equation once a group per term would take more than
+// one wave of resident blocks.
 bool miller_per_equation(uint64_t terms) {
     static const uint64_t wave = [] {
         int blocks = 0;
-        DV_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k_miller_multi, 128, 0));
-        return (uint64_t)sm_count() * (uint64_t)std::max(1, blocks) * GROUPS_PER_BLOCK;
+        DV_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k_miller_multi<1>, THREADS, SM_BYTES<1>));
+        return (uint64_t)sm_count() * (uint64_t)std::max(1, blocks) * GROUPS_PER_BLOCK<1>;
     }();
     return terms > wave;
 }
@@ -705,13 +788,12 @@ uint64_t* upload_offsets(Backend& b, const uint64_t* offsets, uint64_t equations
 // Final exponentiation of the Miller values in mil (one per term, folded per
 // equation by the device offsets d_off; one per equation when d_off is
 // null), verdicts / GT elements back to the host.
-void finish_equations(Backend& b, Fq2* mil, const uint64_t* d_off, uint64_t equations, uint8_t* verdicts,
+void finish_equations(Backend& b, const Fq* mil, const uint64_t* d_off, uint64_t equations, uint8_t* verdicts,
                       uint8_t* gt, const uint32_t* bad, const std::vector<uint64_t>* g2_first, cudaStream_t st) {
     // GT elements first (16-byte aligned stores), then the verdict bytes
     uint8_t* d_gt = b.out_buf.as<uint8_t>(equations * ((gt ? 384 : 0) + 1));
     uint8_t* d_out = d_gt + (gt ? 384 * equations : 0);
-    k_final_exp<<<group_blocks(equations), 128, 0, st>>>(mil, d_off, equations, d_out, gt ? d_gt : nullptr);
-    DV_LAUNCH();
+    launch_final_exp(mil, d_off, equations, d_out, gt ? d_gt : nullptr, st);
     uint32_t hbad[2];
     DV_CUDA(cudaMemcpyAsync(hbad, bad, sizeof(hbad), cudaMemcpyDeviceToHost, st));
     DV_CUDA(cudaStreamSynchronize(st));
@@ -779,23 +861,17 @@ void pairing_run(Backend& b, const uint8_t* g1, const uint8_t* g2, uint64_t term
     convert_points<Fq>(d_in, p, terms, bad, st);
     convert_points<Fq2>(d_in + 64 * terms, q, g2_count, bad + 1, st);
     uint64_t* d_off = upload_offsets(b, offsets, equations, st);
-    Fq2* mil = b.aux.as<Fq2>(6 * std::max<uint64_t>(1, std::max(terms, equations)));
+    Fq* mil = b.aux.as<Fq>(12 * std::max<uint64_t>(1, std::max(terms, equations)));
     if (prepared) {
         PairingState& ps = pairing_state(b);
         Line* lines = ps.lines.as<Line>((uint64_t)LINES * nq);
         uint32_t* qinf = ps.inf.as<uint32_t>(nq);
         uint32_t* d_qidx = ps.qidx.as<uint32_t>(terms);
         DV_CUDA(cudaMemcpyAsync(d_qidx, qidx.data(), 4 * terms, cudaMemcpyHostToDevice, st));
-        k_prepare<<<group_blocks(nq), 128, 0, st>>>(q, nq, lines, qinf);
-        DV_LAUNCH();
-        if (multi)
-            k_miller_multi<<<group_blocks(equations), 128, 0, st>>>(p, d_qidx, qinf, lines, d_off, equations, mil);
-        else
-            k_miller_multi<<<group_blocks(terms), 128, 0, st>>>(p, d_qidx, qinf, lines, nullptr, terms, mil);
-        DV_LAUNCH();
+        launch_prepare(q, nq, lines, qinf, st);
+        launch_miller_multi(p, d_qidx, qinf, lines, multi ? d_off : nullptr, multi ? equations : terms, mil, st);
     } else if (terms) {
-        k_miller<<<group_blocks(terms), 128, 0, st>>>(p, q, terms, mil);
-        DV_LAUNCH();
+        launch_miller(p, q, terms, mil, st);
     }
     finish_equations(b, mil, prepared && multi ? nullptr : d_off, equations, verdicts, gt, bad,
                      prepared ? &first : nullptr, st);
@@ -813,8 +889,7 @@ uint64_t pairing_prepared_bytes() { return (uint64_t)LINES * sizeof(Line); }
 void pairing_prepare_device(const G2A* q, uint64_t nq, void* lines, uint32_t* qinf, cudaStream_t st) {
     if (!nq) return;
     if (nq > PREP_MAX) throw InvalidArgument("too many distinct G2 points in one check");
-    k_prepare<<<group_blocks(nq), 128, 0, st>>>(q, nq, static_cast<Line*>(lines), qinf);
-    DV_LAUNCH();
+    launch_prepare(q, nq, static_cast<Line*>(lines), qinf, st);
 }
 
 // Pairing-product checks over prepared G2 points, with no host
@@ -828,18 +903,11 @@ void pairing_check_prepared(Backend& b, const G1A* p, uint64_t terms, const void
                             cudaStream_t st) {
     if (!equations) return;
     const Line* ln = static_cast<const Line*>(lines);
-    Fq2* mil = b.aux.as<Fq2>(6 * std::max<uint64_t>(1, std::max(terms, equations)));
+    Fq* mil = b.aux.as<Fq>(12 * std::max<uint64_t>(1, std::max(terms, equations)));
     const bool multi = miller_per_equation(terms);
-    if (multi) {
-        k_miller_multi<<<group_blocks(equations), 128, 0, st>>>(p, d_qidx, qinf, ln, d_off, equations, mil);
-        DV_LAUNCH();
-    } else if (terms) {
-        k_miller_multi<<<group_blocks(terms), 128, 0, st>>>(p, d_qidx, qinf, ln, nullptr, terms, mil);
-        DV_LAUNCH();
-    }
-    k_final_exp<<<group_blocks(equations), 128, 0, st>>>(mil, multi ? nullptr : d_off, equations, d_verdicts,
-                                                         nullptr);
-    DV_LAUNCH();
+    if (multi) launch_miller_multi(p, d_qidx, qinf, ln, d_off, equations, mil, st);
+    else if (terms) launch_miller_multi(p, d_qidx, qinf, ln, nullptr, terms, mil, st);
+    launch_final_exp(mil, multi ? nullptr : d_off, equations, d_verdicts, nullptr, st);
 }
 
 // The same checks with the nq G2 points of q prepared first (into the
@@ -904,9 +972,7 @@ extern "C" int dvgpu_bn254_g2_prepare(void* opaque, const uint8_t* g2, size_t n,
         DV_CUDA(cudaMemsetAsync(bad, 0xff, sizeof(uint32_t), st));
         G2A* q = pg->points.as<G2A>(n);
         convert_points<Fq2>(d_in, q, n, bad, st);
-        k_prepare<<<group_blocks(n), 128, 0, st>>>(q, n, pg->lines.as<Line>((uint64_t)LINES * n),
-                                                   pg->inf.as<uint32_t>(n));
-        DV_LAUNCH();
+        launch_prepare(q, n, pg->lines.as<Line>((uint64_t)LINES * n), pg->inf.as<uint32_t>(n), st);
         const uint32_t first_bad = read_err_word(b, bad, st);
         if (first_bad != 0xffffffffu) throw InvalidArgument("invalid G2 point at index " + std::to_string(first_bad));
         const uint64_t h = b.next_handle++;
@@ -944,20 +1010,14 @@ extern "C" int dvgpu_bn254_pairing_check_prepared(void* opaque, const uint8_t* g
         DV_CUDA(cudaMemsetAsync(bad, 0xff, 2 * sizeof(uint32_t), st));
         convert_points<Fq>(d_in, p, terms, bad, st);
         uint64_t* d_off = upload_offsets(b, offsets, equations, st);
-        Fq2* mil = b.aux.as<Fq2>(6 * std::max<uint64_t>(1, std::max(terms, equations)));
+        Fq* mil = b.aux.as<Fq>(12 * std::max<uint64_t>(1, std::max(terms, equations)));
         uint32_t* d_qidx = ps.qidx.as<uint32_t>(std::max<uint64_t>(1, terms));
         if (terms) DV_CUDA(cudaMemcpyAsync(d_qidx, q_index, 4 * terms, cudaMemcpyHostToDevice, st));
         const bool multi = miller_per_equation(terms);
-        if (multi) {
-            // with no terms every equation's value is one (the kernel reads only the offsets)
-            k_miller_multi<<<group_blocks(equations), 128, 0, st>>>(p, d_qidx, pg.inf.view<uint32_t>(),
-                                                                   pg.lines.view<Line>(), d_off, equations, mil);
-            DV_LAUNCH();
-        } else if (terms) {
-            k_miller_multi<<<group_blocks(terms), 128, 0, st>>>(p, d_qidx, pg.inf.view<uint32_t>(),
-                                                               pg.lines.view<Line>(), nullptr, terms, mil);
-            DV_LAUNCH();
-        }
+        // with no terms every equation's value is one (the kernels read only the offsets)
+        if (terms)
+            launch_miller_multi(p, d_qidx, pg.inf.view<uint32_t>(), pg.lines.view<Line>(), multi ? d_off : nullptr,
+                                multi ? equations : terms, mil, st);
         finish_equations(b, mil, multi ? nullptr : d_off, equations, verdicts, nullptr, bad, nullptr, st);
     });
 }
