@@ -329,3 +329,30 @@ def test_resident_host_msm(backend, oracle, dv):
         assert backend.msm_resident_host(h, sc) == expect  # owner still healthy
     finally:
         backend.release_bases(h)
+
+
+@pytest.mark.parametrize("n", [230001, 420000])
+@pytest.mark.parametrize("digits", ["uniform", "one value"])
+def test_g1_msm_pairwise_levels(backend, oracle, n, digits):
+    """Lists long enough for one and for two pairwise levels, over 64 distinct
+    bases in turn (with infinity and opposite points), so that buckets are full
+    of equal, opposite and absent points; with one scalar everywhere a bucket
+    spans many lanes.  Expected: the 64-term sum of the collected scalars."""
+    r = 0x30644E72E131A029B85045B68181585D2833E84879B9709143E1F593F0000001
+    q = 0x30644E72E131A029B85045B68181585D97816A916871CA8D3C208C16D87CFD47
+    half = oracle.fixed_base_g1(oracle.uniform_fr(6101, 32))
+    bases = [half[64 * i:64 * i + 64] for i in range(32)]
+    bases += [p[:32] + (q - int.from_bytes(p[32:], "little")).to_bytes(32, "little") for p in bases]
+    bases[5] = bases[44] = bytes(64)
+    if digits == "uniform":
+        sc = bytearray(oracle.uniform_fr(6102, n))
+        for i in range(0, n, 11):
+            sc[32 * i:32 * i + 32] = bytes(32)
+        sc = bytes(sc)
+    else:
+        sc = oracle.uniform_fr(6103, 1) * n
+    pts = (b"".join(bases) * (n // 64 + 1))[:64 * n]
+    limbs = np.frombuffer(sc, dtype="<u4").reshape(n, 8).astype(np.uint64)
+    sums = [sum(int(x) << (32 * k) for k, x in enumerate(limbs[i::64].sum(axis=0))) % r for i in range(64)]
+    expect = oracle.msm_g1(b"".join(bases), b"".join(x.to_bytes(32, "little") for x in sums))
+    assert backend.msm(pts, sc) == expect
