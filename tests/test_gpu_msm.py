@@ -356,3 +356,25 @@ def test_g1_msm_pairwise_levels(backend, oracle, n, digits):
     sums = [sum(int(x) << (32 * k) for k, x in enumerate(limbs[i::64].sum(axis=0))) % r for i in range(64)]
     expect = oracle.msm_g1(b"".join(bases), b"".join(x.to_bytes(32, "little") for x in sums))
     assert backend.msm(pts, sc) == expect
+
+
+@pytest.mark.parametrize("g2", [False, True])
+@pytest.mark.parametrize("n", [1, 9, 300, 2500, 20000])
+def test_msm_repeated_scalars(backend, oracle, n, g2):
+    """One scalar everywhere over four bases in turn: every window is one
+    bucket over all slices, merged by a quad, a warp or a block as n grows, of
+    equal and opposite partial sums; digits shared among up to W threads."""
+    q = 0x30644E72E131A029B85045B68181585D97816A916871CA8D3C208C16D87CFD47
+    size, fixed = (128, oracle.fixed_base_g2) if g2 else (64, oracle.fixed_base_g1)
+    p = fixed(oracle.uniform_fr(6201, 1))
+    neg = p[:size // 2] + b"".join((-int.from_bytes(p[i:i + 32], "little") % q).to_bytes(32, "little")
+                                   for i in range(size // 2, size, 32))
+    bases = [p, p, neg, fixed(oracle.uniform_fr(6202, 1))]
+    pts = (b"".join(bases) * (n // 4 + 1))[:size * n]
+    run = backend.msm_g2_host if g2 else backend.msm
+    ref = oracle.msm_g2 if g2 else oracle.msm_g1
+    r = 0x30644E72E131A029B85045B68181585D2833E84879B9709143E1F593F0000001
+    for s in (1, r - 1, int.from_bytes(oracle.uniform_fr(6203, 1), "little")):
+        counts = [(n + 3 - i) // 4 * s % r for i in range(4)]
+        expect = ref(b"".join(bases), b"".join(c.to_bytes(32, "little") for c in counts))
+        assert run(pts, s.to_bytes(32, "little") * n) == expect, s

@@ -175,6 +175,13 @@ struct XYZZ {
 };
 
 // ------------------------------------------------------------- warp helpers
+DV_INL Fq shfl_xor(const Fq& a, int m) {
+    Fq r;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) r.v[i] = __shfl_xor_sync(0xffffffffu, a.v[i], m);
+    return r;
+}
+DV_INL Fq2 shfl_xor(const Fq2& a, int m) { return {shfl_xor(a.c0, m), shfl_xor(a.c1, m)}; }
 DV_INL Fq shfl_up(const Fq& a, int d) {
     Fq r;
 #pragma unroll
@@ -220,6 +227,62 @@ DV_INL F warp_batch_inverse(const F& x) {
     if (lane == 31) excl_suf = F::one();
     return F::mul(total_inv, F::mul(excl_pre, excl_suf));
 }
+
+// Points held by four lanes, lane r of an aligned quad one coordinate (x, y,
+// zz, zzz): an addition is four dependent products instead of a lane's
+// fourteen, a doubling three instead of nine, for chains of few points (a
+// quarter more multiply-adds a point when lanes are not free).  Every lane of
+// the warp takes part; quads without work hold infinity.
+template <class F>
+struct Quad {
+    F c;
+
+    DV_INL static int role() { return (int)(threadIdx.x & 3); }
+    DV_INL static F from(const F& a, int r) { return shfl_idx(a, (int)(threadIdx.x & 28) + r); }
+    DV_INL static bool flag(bool b, int r) { return __shfl_sync(0xffffffffu, (int)b, (int)(threadIdx.x & 28) + r) != 0; }
+    DV_INL static F inf() { return role() < 2 ? F::one() : F::zero(); }
+    DV_INL static F pick(int r, const F& a0, const F& a1, const F& a2, const F& a3) {
+        return r == 0 ? a0 : r == 1 ? a1 : r == 2 ? a2 : a3;
+    }
+
+    static __device__ __noinline__ F dbl(F p) {
+        const int r = role();
+        const F u = F::dbl(p);                             // lane 1: U = 2 Y
+        const F m1 = F::sqr(r == 1 ? u : p);               // X^2, V = U^2
+        const F v = from(m1, 1), xx = from(m1, 0);
+        const F m = F::add(F::dbl(xx), xx);
+        const F m2 = F::mul(pick(r, p, u, p, m), r == 3 ? m : v);  // S, W, ZZ3, M^2
+        const F s = from(m2, 0), w = from(m2, 1);
+        const F x3 = F::sub(from(m2, 3), F::dbl(s));
+        const F m3 = F::mul(r == 0 ? m : p, r == 0 ? F::sub(s, x3) : w);  // M (S - X3), W Y, -, ZZZ3
+        const F y3 = F::sub(from(m3, 0), m3);
+        return pick(r, x3, y3, m2, m3);
+    }
+    static __device__ __noinline__ F add(F p, F q) {
+        const int r = role();
+        const bool pi = flag(p.is_zero(), 2), qi = flag(q.is_zero(), 2);
+        const F t = F::mul(p, shfl_xor(q, 2));             // U1, S1, U2, S2
+        const F o = shfl_xor(t, 2);
+        const F d = r < 2 ? F::sub(o, t) : F::sub(t, o);   // P on lanes 0, 2; R on 1, 3
+        const bool same_x = flag(d.is_zero(), 0), same_y = flag(d.is_zero(), 1);
+        const F m2 = F::mul(r < 2 ? d : p, r < 2 ? d : q);  // PP, R^2, ZZ1 ZZ2, ZZZ1 ZZZ2
+        const F pp = from(m2, 0), pv = from(d, 0);
+        const F m3 = F::mul(r == 0 ? t : r == 1 ? pv : m2, pp);  // Q, PPP, ZZ3
+        const F qv = from(m3, 0), ppp = from(m3, 1);
+        const F x3 = F::sub(F::sub(from(m2, 1), ppp), F::dbl(qv));
+        const F s1 = from(t, 1);
+        const F m4 = F::mul(pick(r, s1, d, m2, m2), r == 1 ? F::sub(qv, x3) : ppp);  // S1 PPP, R (Q - X3), -, ZZZ3
+        const F y3 = F::sub(m4, from(m4, 0));
+        F out = pick(r, x3, y3, m3, m4);
+        const bool twice = same_x && same_y && !pi && !qi;
+        if (__any_sync(0xffffffffu, twice)) {
+            const F two = dbl(p);
+            if (twice) out = two;
+        }
+        if (same_x && !same_y && !pi && !qi) out = inf();
+        return pi ? q : qi ? p : out;
+    }
+};
 
 typedef Affine<Fq> G1A;
 typedef XYZZ<Fq> G1X;

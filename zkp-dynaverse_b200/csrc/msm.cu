@@ -26,6 +26,18 @@ DV_INL uint32_t window_raw(const uint32_t* s, int bit, int c) {
     return v & ((1u << c) - 1u);
 }
 
+// Carry into window w of the signed recoding (digits in (-B, B], B =
+// 2^(c-1); a window above B goes negative and carries): decided by the next
+// lower window unless that is exactly B.
+DV_INL uint32_t carry_into(const uint32_t* s, int w, int c) {
+    const uint32_t B = 1u << (c - 1);
+    for (int v = w - 1; v >= 0; --v) {
+        const uint32_t d = window_raw(s, v * c, c);
+        if (d != B) return d > B ? 1u : 0u;
+    }
+    return 0;
+}
+
 DV_INL void load_scalar(const uint32_t* scalars, uint32_t i, uint32_t* s) {
     const uint4* q = reinterpret_cast<const uint4*>(scalars + 8ull * i);
     const uint4 a = q[0], b = q[1];
@@ -51,7 +63,18 @@ DV_INL void locate(const SetMap& m, uint32_t i, uint32_t& set, uint32_t& sidx, u
     pidx = m.term_point ? m.term_point[i] : m.prefix ? rel : sidx;
 }
 
-// 1. Histogram of signed digits.
+// Windows [w0, w1) of this block: blockIdx.y of gridDim.y even shares.
+DV_INL void window_share(int W, int& w0, int& w1) {
+    const int per = (W + (int)gridDim.y - 1) / (int)gridDim.y;
+    w0 = min(W, (int)blockIdx.y * per);
+    w1 = min(W, w0 + per);
+}
+
+// 1. Histogram of signed digits.  Few scalars leave the GPU idle on W
+// dependent atomics each, so their windows are shared among gridDim.y threads
+// (the carry into a thread's first window is found by carry_into): 1000
+// scalars of 32 windows, histogram and scatter, 39 us with one thread a
+// scalar, 10 us with one a window.
 template <bool PRE>
 __global__ void k_hist(const uint32_t* __restrict__ scalars, uint32_t n, const SetMap m, int c, int W,
                        uint32_t* __restrict__ counts, uint32_t* __restrict__ first_bad) {
@@ -70,9 +93,12 @@ __global__ void k_hist(const uint32_t* __restrict__ scalars, uint32_t n, const S
     const uint32_t base = PRE ? set * B : set * (uint32_t)W * B;
     const uint32_t active = __activemask();
     const uint32_t lane = threadIdx.x & 31;
-    uint32_t carry = 0;
-    for (int w = 0; w < W; ++w) {
-        const uint32_t d = window_raw(s, w * c, c) + carry;
+    const uint32_t* words = scalars + 8ull * sidx;
+    int w0, w1;
+    window_share(W, w0, w1);
+    uint32_t carry = carry_into(words, w0, c);
+    for (int w = w0; w < w1; ++w) {
+        const uint32_t d = window_raw(words, w * c, c) + carry;
         const bool neg = d > B;
         const uint32_t mag = neg ? full - d : d;
         carry = neg ? 1u : 0u;
@@ -183,9 +209,12 @@ __global__ void k_scatter(const uint32_t* __restrict__ scalars, uint32_t n, cons
     const uint32_t base = PRE ? set * B : set * (uint32_t)W * B;
     const uint32_t active = __activemask();
     const uint32_t lane = threadIdx.x & 31;
-    uint32_t carry = 0;
-    for (int w = 0; w < W; ++w) {
-        const uint32_t d = window_raw(s, w * c, c) + carry;
+    const uint32_t* words = scalars + 8ull * sidx;
+    int w0, w1;
+    window_share(W, w0, w1);
+    uint32_t carry = carry_into(words, w0, c);
+    for (int w = w0; w < w1; ++w) {
+        const uint32_t d = window_raw(words, w * c, c) + carry;
         const bool neg = d > B;
         const uint32_t mag = neg ? full - d : d;
         carry = neg ? 1u : 0u;
@@ -614,54 +643,90 @@ __global__ void __launch_bounds__(128, PAIR_BLOCKS) k_pair_level(const AccumChun
 
 // 5. Merge partials of buckets that span slices.  The owner of bucket g is
 // the slice whose tail holds g; the following slices hold g in their heads.
-// Chains of more than FIX_SHORT heads (a bucket spanning many slices: skewed
-// digits) are queued for k_fixup_long, which merges them with a block-wide
-// tree instead of one serial walk.
-constexpr uint32_t FIX_SHORT = 32;
+// A lane quad per slice adds up to FIX_SHORT heads in turn (most buckets are
+// cut once).  Longer chains (skewed digits, few buckets) are queued: k_fixup_long
+// gives each a warp, eight quads and a three-step tree, and those of more
+// than FIX_WARP heads a block.  A merge is 2.5 us (G2: 5) where a thread's
+// took 6: 1000 points 33 -> 9 us; limits of 4, 8 and 16 measured the same.
+constexpr uint32_t FIX_SHORT = 8, FIX_WARP = 256;
 
 template <class F>
-__global__ void k_fixup(const int* __restrict__ pgid, const XYZZ<F>* __restrict__ ppt, uint32_t T,
+__global__ void __launch_bounds__(256) k_fixup(const int* __restrict__ pgid, const XYZZ<F>* __restrict__ ppt, uint32_t T,
                         XYZZ<F>* __restrict__ buckets, uint32_t* __restrict__ long_list,
                         uint32_t* __restrict__ long_count, const AccumChunk* __restrict__ chunk) {
     if (chunk) buckets += chunk->b0;
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= T) return;
-    const int g = pgid[2 * t + 1];
-    if (g < 0) return;
-    uint32_t end = t + 1;
-    while (end < T && pgid[2 * end] == g && end - t <= FIX_SHORT) ++end;
-    if (end < T && pgid[2 * end] == g) {
-        long_list[atomicAdd(long_count, 1u)] = t;
-        return;
-    }
-    XYZZ<F> acc = ppt[2 * t + 1];
-    for (uint32_t k = t + 1; k < end; ++k) acc = XYZZ<F>::add(acc, ppt[2 * k]);
-    buckets[g] = acc;
+    const uint32_t t = (blockIdx.x * blockDim.x + threadIdx.x) >> 2, r = threadIdx.x & 3;
+    const int g = t < T ? pgid[2 * t + 1] : -1;
+    uint32_t heads = 0;
+    if (g >= 0)
+        while (heads <= FIX_SHORT && t + 1 + heads < T && pgid[2 * (t + 1 + heads)] == g) ++heads;
+    const bool queued = heads > FIX_SHORT;
+    if (queued && r == 0) long_list[atomicAdd(long_count, 1u)] = t;
+    if (queued || g < 0) heads = 0;
+    const F* parts = reinterpret_cast<const F*>(ppt);
+    F acc = g >= 0 ? parts[(size_t)(2 * t + 1) * 4 + r] : Quad<F>::inf();
+    for (uint32_t k = 1; __any_sync(0xffffffffu, k <= heads); ++k)
+        acc = Quad<F>::add(acc, k <= heads ? parts[(size_t)(2 * (t + k)) * 4 + r] : Quad<F>::inf());
+    if (g >= 0 && !queued) reinterpret_cast<F*>(buckets)[(size_t)g * 4 + r] = acc;
 }
 
-template <class F, int TH>
-__global__ void __launch_bounds__(TH) k_fixup_long(const int* __restrict__ pgid, const XYZZ<F>* __restrict__ ppt,
+// The sum over the quads of a group of lanes: quad 0 ends with it.
+template <class F>
+DV_INL F quads_sum_warp(F acc) {
+#pragma unroll 1
+    for (int d = 16; d >= 4; d >>= 1) acc = Quad<F>::add(acc, shfl_xor(acc, d));
+    return acc;
+}
+
+template <class F>
+__global__ void __launch_bounds__(256) k_fixup_long(const int* __restrict__ pgid, const XYZZ<F>* __restrict__ ppt,
                                                    uint32_t T, XYZZ<F>* __restrict__ buckets,
                                                    const uint32_t* __restrict__ long_list,
                                                    const uint32_t* __restrict__ long_count,
                                                    const AccumChunk* __restrict__ chunk) {
-    __shared__ XYZZ<F> sh[TH];
+    __shared__ F warp_sum[8][4];
+    __shared__ uint32_t huge[8];
     if (chunk) buckets += chunk->b0;
-    const uint32_t nlong = *long_count;
-    for (uint32_t item = blockIdx.x; item < nlong; item += gridDim.x) {
-        const uint32_t t0 = long_list[item];
-        const int g = pgid[2 * t0 + 1];
-        XYZZ<F> acc = threadIdx.x == 0 ? ppt[2 * t0 + 1] : XYZZ<F>::inf();
-        // the heads of g are contiguous from t0 + 1: stop at the first other key
-        for (uint32_t k = t0 + 1 + threadIdx.x; k < T && pgid[2 * k] == g; k += TH)
-            acc = XYZZ<F>::add(acc, ppt[2 * k]);
-        sh[threadIdx.x] = acc;
+    const uint32_t nlong = *long_count, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, r = threadIdx.x & 3;
+    const F* parts = reinterpret_cast<const F*>(ppt);
+    F* out = reinterpret_cast<F*>(buckets);
+    // heads of g at positions from + step k, while they are g's (contiguous from t0 + 1)
+    const auto add_heads = [&](F acc, int g, uint32_t from, uint32_t step) {
+        for (uint32_t k = from;; k += step) {
+            const bool have = k < T && pgid[2 * k] == g;
+            if (!__any_sync(0xffffffffu, have)) return acc;
+            acc = Quad<F>::add(acc, have ? parts[(size_t)(2 * k) * 4 + r] : Quad<F>::inf());
+        }
+    };
+    for (uint32_t base = blockIdx.x * 8; base < nlong; base += gridDim.x * 8) {
+        const uint32_t item = base + warp;
+        bool is_huge = false;
+        if (item < nlong) {
+            const uint32_t t0 = long_list[item], far = t0 + 1 + FIX_WARP;
+            const int g = pgid[2 * t0 + 1];
+            is_huge = far < T && pgid[2 * far] == g;
+            if (!is_huge) {
+                F acc = lane < 4 ? parts[(size_t)(2 * t0 + 1) * 4 + r] : Quad<F>::inf();
+                acc = quads_sum_warp<F>(add_heads(acc, g, t0 + 1 + (lane >> 2), 8));
+                if (lane < 4) out[(size_t)g * 4 + r] = acc;
+            }
+        }
+        if (lane == 0) huge[warp] = is_huge ? item : 0xffffffffu;
         __syncthreads();
-        for (int d = TH / 2; d > 0; d >>= 1) {
-            if ((int)threadIdx.x < d) sh[threadIdx.x] = XYZZ<F>::add(sh[threadIdx.x], sh[threadIdx.x + d]);
+        for (int h = 0; h < 8; ++h) {
+            if (huge[h] == 0xffffffffu) continue;
+            const uint32_t t0 = long_list[huge[h]];
+            const int g = pgid[2 * t0 + 1];
+            F acc = threadIdx.x < 4 ? parts[(size_t)(2 * t0 + 1) * 4 + r] : Quad<F>::inf();
+            acc = quads_sum_warp<F>(add_heads(acc, g, t0 + 1 + (threadIdx.x >> 2), 64));
+            if (lane < 4) warp_sum[warp][r] = acc;
+            __syncthreads();
+            if (warp == 0) {
+                acc = quads_sum_warp<F>(warp_sum[lane >> 2][r]);
+                if (lane < 4) out[(size_t)g * 4 + r] = acc;
+            }
             __syncthreads();
         }
-        if (threadIdx.x == 0) buckets[g] = sh[0];
         __syncthreads();
     }
 }
@@ -691,15 +756,6 @@ DV_INL XYZZ<F> wdbl(const XYZZ<F>& p) {
     if constexpr (sizeof(F) == sizeof(Fq)) return XYZZ<F>::dbl_paired(p);
     else return XYZZ<F>::dbl(p);
 }
-template <class F>
-DV_INL XYZZ<F> shfl_down_xyzz(const XYZZ<F>& p, int d) {
-    return {shfl_down(p.x, d), shfl_down(p.y, d), shfl_down(p.zz, d), shfl_down(p.zzz, d)};
-}
-template <class F>
-DV_INL XYZZ<F> shfl_idx_xyzz(const XYZZ<F>& p, int l) {
-    return {shfl_idx(p.x, l), shfl_idx(p.y, l), shfl_idx(p.zz, l), shfl_idx(p.zzz, l)};
-}
-
 // Level 1: one segment of s buckets per thread.
 template <class F>
 __global__ void __launch_bounds__(128) k_segments(const XYZZ<F>* __restrict__ buckets, const uint32_t* __restrict__ offsets,
@@ -722,78 +778,54 @@ __global__ void __launch_bounds__(128) k_segments(const XYZZ<F>* __restrict__ bu
     seg_v[tid] = R;
 }
 
-// Upper levels: blocks of P pairs (G = P), windows of S pairs; S <= P is the
-// last level (one block per window, its U' is S_w).  Suffix sums of V by
-// warp shuffles (five rounds in a warp, three across the block's warp
-// totals), then the block sum of U + Suf_{+1} the same way: about 18
-// dependent additions and three barriers per block, then log2 P doublings
-// for V'.  A block's time is this chain's latency (measured the same as a
-// shared-memory Hillis-Steele scan and tree of equal depth), so the
-// levels cost about one block latency per wave of blocks: 16-bucket
-// segments for 2^19 buckets keep the first upper level to one wave.
-template <class F, int P>
-__global__ void __launch_bounds__(P) k_wlevel(const XYZZ<F>* __restrict__ u_in, const XYZZ<F>* __restrict__ v_in,
-                                              uint32_t S, XYZZ<F>* __restrict__ u_out, XYZZ<F>* __restrict__ v_out) {
-    constexpr int NWARP = P / 32;
-    static_assert(NWARP >= 1 && NWARP <= 32 && (NWARP & (NWARP - 1)) == 0, "block of 32..1024 threads, power of 2");
-    __shared__ XYZZ<F> warp_v[NWARP], warp_later[NWARP], warp_x[NWARP];
-    __shared__ XYZZ<F> block_v;
-    const uint32_t nblk = S > (uint32_t)P ? S / P : 1u;
+// Upper levels: blocks of WTREE pairs (G = WTREE), windows of S pairs; S <=
+// WTREE is the last level (one block per window, its U' is S_w).  A binary
+// tree: pairs 2j and 2j + 1 give
+//      U = U_a + U_b + V_b,   V = 2 (V_a + V_b),
+// one lane quad for each of the two, so a tree level is two dependent point
+// operations whatever the number of pairs, and V ends multiplied by G.  A
+// window of S pairs is the latency of 2 log2(S) operations of 2.5 us (G2: 5 us),
+// where suffix scans by one lane a point took 26 operations of 6 us a level.
+// All upper levels of one MSM: 2^18 buckets, 310 -> 158 us; 1000 points, 115 ->
+// 49 us; G2, 2^16 points, 627 -> 392 us.
+constexpr int WTREE = 64;
+template <class F>
+__global__ void __launch_bounds__(256) k_wtree(const XYZZ<F>* __restrict__ u_in, const XYZZ<F>* __restrict__ v_in,
+                                               uint32_t S, XYZZ<F>* __restrict__ u_out, XYZZ<F>* __restrict__ v_out) {
+    __shared__ F sh[2 * WTREE][4];  // U, then V
+    const uint32_t nblk = S > (uint32_t)WTREE ? S / WTREE : 1u;
     const uint32_t w = blockIdx.x / nblk, k = blockIdx.x % nblk;
-    const uint32_t width = S < (uint32_t)P ? S : (uint32_t)P;
-    const uint32_t t = threadIdx.x;
-    const int lane = (int)(t & 31), warp = (int)(t >> 5);
-    const size_t idx = (size_t)w * S + (size_t)k * P + t;
-    const bool live = t < width;
-    // inclusive suffix sums of V inside the warp
-    XYZZ<F> sv = live ? v_in[idx] : XYZZ<F>::inf();
-#pragma unroll 1
-    for (int d = 1; d < 32; d <<= 1) {
-        const XYZZ<F> o = shfl_down_xyzz(sv, d);
-        if (lane + d < 32) sv = wadd<F>(sv, o);
-    }
-    if (lane == 0) warp_v[warp] = sv;
-    __syncthreads();
-    // suffix sums over the warp totals (warp 0): later warps' V for every warp
-    if (warp == 0) {
-        XYZZ<F> c = lane < NWARP ? warp_v[lane] : XYZZ<F>::inf();
-#pragma unroll 1
-        for (int d = 1; d < NWARP; d <<= 1) {
-            const XYZZ<F> o = shfl_down_xyzz(c, d);
-            if (lane + d < NWARP) c = wadd<F>(c, o);
-        }
-        const XYZZ<F> after = shfl_down_xyzz(c, 1);
-        if (lane < NWARP) warp_later[lane] = lane + 1 < NWARP ? after : XYZZ<F>::inf();
-        if (lane == 0) block_v = c;
+    const uint32_t width = S < (uint32_t)WTREE ? S : (uint32_t)WTREE;
+    const size_t first = ((size_t)w * S + (size_t)k * WTREE) * 4;
+    for (uint32_t i = threadIdx.x; i < 4 * width; i += 256) {
+        (&sh[0][0])[i] = reinterpret_cast<const F*>(u_in)[first + i];
+        (&sh[WTREE][0])[i] = reinterpret_cast<const F*>(v_in)[first + i];
     }
     __syncthreads();
-    // Suf_{t+1} + U_t
-    const XYZZ<F> nxt = shfl_down_xyzz(sv, 1);
-    XYZZ<F> x = wadd<F>(lane < 31 ? nxt : XYZZ<F>::inf(), warp_later[warp]);
-    if (live) x = wadd<F>(x, u_in[idx]);
-    // block sum: butterfly in the warp, then the warp sums in warp 0
-#pragma unroll 1
-    for (int d = 16; d >= 1; d >>= 1) {
-        const XYZZ<F> o = shfl_down_xyzz(x, d);
-        if (lane < d) x = wadd<F>(x, o);
+    const uint32_t quad = threadIdx.x >> 2, r = threadIdx.x & 3;
+    for (uint32_t m = width / 2; m >= 1; m >>= 1) {
+        // U on the first quads, V on the next, never both in one warp
+        const uint32_t v0 = m < 8 ? 8 : m;
+        const bool is_u = quad < m, is_v = quad >= v0 && quad < v0 + m;
+        const uint32_t j = is_u ? quad : quad - v0;
+        const bool warp_u = (threadIdx.x >> 5) * 8 < m;
+        const bool warp_v = !warp_u && (threadIdx.x >> 5) * 8 < v0 + m;
+        F s = Quad<F>::inf();
+        if (warp_u || warp_v) {
+            const F* x = &sh[is_v ? WTREE : 0][0];
+            const bool live = is_u || is_v;
+            s = Quad<F>::add(live ? x[(2 * j) * 4 + r] : Quad<F>::inf(), live ? x[(2 * j + 1) * 4 + r] : Quad<F>::inf());
+            if (warp_u) s = Quad<F>::add(s, is_u ? sh[WTREE + 2 * j + 1][r] : Quad<F>::inf());
+            else s = Quad<F>::dbl(s);
+        }
+        __syncthreads();
+        if (is_u) sh[j][r] = s;
+        if (is_v) sh[WTREE + j][r] = s;
+        __syncthreads();
     }
-    if (lane == 0) warp_x[warp] = x;
-    __syncthreads();
-    if (warp == 0) {
-        XYZZ<F> y = lane < NWARP ? warp_x[lane] : XYZZ<F>::inf();
-#pragma unroll 1
-        for (int d = NWARP / 2; d >= 1; d >>= 1) {
-            const XYZZ<F> o = shfl_down_xyzz(y, d);
-            if (lane < d) y = wadd<F>(y, o);
-        }
-        if (lane == 0) {
-            u_out[blockIdx.x] = y;
-            if (nblk > 1) {
-                XYZZ<F> vsum = block_v;
-                for (int i = 0; i < __builtin_ctz((unsigned)P); ++i) vsum = wdbl<F>(vsum);  // V' = P sum V
-                v_out[blockIdx.x] = vsum;
-            }
-        }
+    if (threadIdx.x < 4) {
+        reinterpret_cast<F*>(u_out)[(size_t)blockIdx.x * 4 + r] = sh[0][r];
+        if (nblk > 1) reinterpret_cast<F*>(v_out)[(size_t)blockIdx.x * 4 + r] = sh[WTREE][r];
     }
 }
 
@@ -947,9 +979,9 @@ static int measured_c(uint64_t n) {
 int msm_seg_log(uint64_t all_buckets, uint32_t buckets, int c, bool g1) {
     // Long windows (a precomputed table's single bucket set of 2^18 or more
     // G1 buckets) take 16-bucket segments: fewer upper-level entries for a
-    // modest first level (measured 0.86 instead of 1.06 ms at 2^19 buckets);
-    // shorter windows and G2, whose additions cost three times as much,
-    // keep 8.
+    // modest first level; shorter windows and G2, whose additions cost three
+    // times as much, keep 8 (G1 2^20 points: 3.60 ms with 8 or 16, 3.69 with 4;
+    // G2 2^16 points: 1.80 with 8 or 16, 2.12 with 4).
     int seg_want = (g1 && buckets >= (1u << 18)) ? DV_SEG_LOG + 1 : DV_SEG_LOG;
     // Few buckets in all (sparse updates over a precomputed table, small
     // MSMs): the reduction is a latency chain, so keep about 2^15 first-level
@@ -959,8 +991,8 @@ int msm_seg_log(uint64_t all_buckets, uint32_t buckets, int c, bool g1) {
     // Many buckets in all (a batch of sets over one table, 2^21 buckets or
     // more): longer segments, up to 64 buckets, while at least 2^17
     // first-level threads remain (several waves of k_segments at two blocks
-    // per SM).  Each halving of the segment count halves the first upper
-    // level, whose warp-0 phases and doublings leave most lanes idle.
+    // per SM).  A bucket costs two additions in a segment, a segment four
+    // operations in the tree above.
     int wide = 0;
     while (wide < 6 && (all_buckets >> (wide + 1)) >= (1u << 17)) ++wide;
     seg_want = std::min(std::max(seg_want, wide), room);
@@ -1075,10 +1107,11 @@ void accumulate(MsmWorkspace& ws, const Affine<F>* pts, const uint32_t* d_sorted
         DV_LAUNCH();
         if (!chunk && ws.timeline.enabled) DV_CUDA(cudaEventRecord(ws.timeline.acc_ev[1], st));
         DV_CUDA(cudaMemsetAsync(d_fix_count, 0, sizeof(uint32_t), st));
-        k_fixup<F><<<blocks_for(T, 128), 128, 0, st>>>(d_pgid, d_ppt, T, d_buckets, d_fix_list, d_fix_count, chunk);
+        k_fixup<F><<<blocks_for(4ull * T, 256), 256, 0, st>>>(d_pgid, d_ppt, T, d_buckets, d_fix_list, d_fix_count,
+                                                               chunk);
         DV_LAUNCH();
         // long chains are rare: a small grid loops over the queue
-        k_fixup_long<F, 128><<<std::min<uint32_t>(T / FIX_SHORT + 1, (uint32_t)sm_count()), 128, 0, st>>>(
+        k_fixup_long<F><<<std::min<uint32_t>(T / FIX_SHORT / 8 + 1, (uint32_t)sm_count() * 2), 256, 0, st>>>(
             d_pgid, d_ppt, T, d_buckets, d_fix_list, d_fix_count, chunk);
         DV_LAUNCH();
     };
@@ -1170,8 +1203,11 @@ void msm_enqueue(MsmWorkspace& ws, const Affine<F>* d_points, const uint32_t* d_
         if (tl.enabled) DV_CUDA(cudaEventRecord(tl.ev[k], st));
     };
     mark(0);
-    if (pre) k_hist<true><<<blocks_for(n, 256), 256, 0, st>>>(d_scalars, n, map, c, W, d_counts, d_err);
-    else k_hist<false><<<blocks_for(n, 256), 256, 0, st>>>(d_scalars, n, map, c, W, d_counts, d_err);
+    // threads a scalar: one once the scalars alone fill the GPU
+    const uint32_t share = (uint32_t)std::clamp<uint64_t>((uint64_t)sm_count() * 1024 / n, 1, (uint64_t)W);
+    const dim3 digit_grid(blocks_for(n, 256), share);
+    if (pre) k_hist<true><<<digit_grid, 256, 0, st>>>(d_scalars, n, map, c, W, d_counts, d_err);
+    else k_hist<false><<<digit_grid, 256, 0, st>>>(d_scalars, n, map, c, W, d_counts, d_err);
     DV_LAUNCH();
     mark(1);
     {
@@ -1185,8 +1221,8 @@ void msm_enqueue(MsmWorkspace& ws, const Affine<F>* d_points, const uint32_t* d_
         DV_LAUNCH();
     }
     mark(2);
-    if (pre) k_scatter<true><<<blocks_for(n, 256), 256, 0, st>>>(d_scalars, n, map, c, W, d_cursor, d_sorted);
-    else k_scatter<false><<<blocks_for(n, 256), 256, 0, st>>>(d_scalars, n, map, c, W, d_cursor, d_sorted);
+    if (pre) k_scatter<true><<<digit_grid, 256, 0, st>>>(d_scalars, n, map, c, W, d_cursor, d_sorted);
+    else k_scatter<false><<<digit_grid, 256, 0, st>>>(d_scalars, n, map, c, W, d_cursor, d_sorted);
     DV_LAUNCH();
     mark(3);
 
@@ -1198,7 +1234,6 @@ void msm_enqueue(MsmWorkspace& ws, const Affine<F>* d_points, const uint32_t* d_
     XYZZ<F>* d_lvl_u = d_seg_r + (size_t)NW * S;  // ping-pong buffers of the upper levels
     XYZZ<F>* d_lvl_r = d_lvl_u + (size_t)NW * S;
     XYZZ<F>* d_win = ws.windows.as<XYZZ<F>>(NW);
-    constexpr int P = sizeof(F) == sizeof(Fq) ? 256 : 128;
 
     if (tl.enabled) DV_CUDA(cudaEventRecord(tl.acc_ev[0], st));
     accumulate<F>(ws, pre ? pre->table : d_points, d_sorted, d_offsets, NB, (uint64_t)n * W, d_buckets, st);
@@ -1213,9 +1248,9 @@ void msm_enqueue(MsmWorkspace& ws, const Affine<F>* d_points, const uint32_t* d_
     XYZZ<F>* r2 = d_lvl_r;
     uint32_t len = S;
     for (;;) {
-        const uint32_t nblk = len > (uint32_t)P ? len / P : 1u;
+        const uint32_t nblk = len > (uint32_t)WTREE ? len / WTREE : 1u;
         XYZZ<F>* u_dst = nblk == 1 ? d_win : u2;
-        k_wlevel<F, P><<<NW * nblk, P, 0, st>>>(u, r, len, u_dst, r2);
+        k_wtree<F><<<NW * nblk, 256, 0, st>>>(u, r, len, u_dst, r2);
         DV_LAUNCH();
         if (nblk == 1) break;
         len = nblk;
@@ -1349,14 +1384,10 @@ __global__ void __launch_bounds__(SD_BLOCK) k_sparse_direct(const G1A* __restric
         } else {
             // signed digit of window w (the recoding of k_hist)
             const uint32_t B = 1u << (c - 1), full = 1u << c;
-            uint32_t carry = 0, mag = 0;
-            bool neg = false;
-            for (uint32_t v = 0; v <= w; ++v) {
-                const uint32_t d = window_raw(s, (int)v * c, c) + carry;
-                neg = d > B;
-                mag = neg ? full - d : d;
-                carry = neg ? 1u : 0u;
-            }
+            const uint32_t* words = vals + 8ull * e;
+            const uint32_t d = window_raw(words, (int)w * c, c) + carry_into(words, (int)w, c);
+            const bool neg = d > B;
+            const uint32_t mag = neg ? full - d : d;
             const G1A t = table[ix * (uint64_t)W + w];
             if (mag && !t.is_inf()) {
                 p = XYZZ<Fq>::from_affine(t);

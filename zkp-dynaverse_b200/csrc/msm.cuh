@@ -12,13 +12,15 @@
 //   1. hist     signed c-bit digits of every scalar, count per (set, window, bucket)
 //   2. scan     exclusive prefix sum -> bucket offsets in the sorted list
 //   3. scatter  counting-sort placement of (point index | sign) per digit
-//   4. accum    persistent, perfectly balanced bucket accumulation: each thread
-//               sums a fixed-length slice of the sorted list with XYZZ mixed
-//               additions; buckets cut by a slice boundary leave partials
+//   4. accum    bucket sums.  Long G1 lists are first halved a few times by
+//               affine additions of pairs inside each bucket; then perfectly
+//               balanced accumulation: each thread sums a fixed-length slice
+//               of the list with XYZZ mixed additions; buckets cut by a
+//               slice boundary leave partials
 //   5. fixup    partial sums of buckets that span slices are merged
 //   6. segments per (set, window): running sums over segments of 2^seg_log buckets
-//   7. wlevel   logarithmic-depth levels of the weighted bucket sum (suffix
-//               scan + tree per block), down to one value per (set, window)
+//   7. wtree    binary tree over the weighted segment sums, lane quads per
+//               point, down to one value per (set, window)
 //   8. host     Horner over the windows and normalisation to affine
 // With a table of precomputed window multiples (resident bases), steps 1-7
 // use one bucket set per MSM and step 8 only normalises.
