@@ -378,3 +378,22 @@ def test_msm_repeated_scalars(backend, oracle, n, g2):
         counts = [(n + 3 - i) // 4 * s % r for i in range(4)]
         expect = ref(b"".join(bases), b"".join(c.to_bytes(32, "little") for c in counts))
         assert run(pts, s.to_bytes(32, "little") * n) == expect, s
+
+
+@pytest.mark.parametrize("c", [8, 13])
+def test_sparse_direct_block_edges(backend, oracle, c):
+    """One request around a block's 64 terms and around the direct path's
+    16384 terms, with equal bases, for an even and an odd window width."""
+    n = 1024
+    bases, _ = oracle.srs_g1(4097, n)
+    h = backend.register_bases(bases)
+    try:
+        backend.precompute_bases(h, c)
+        rng = np.random.default_rng(12)
+        windows = -(-255 // c)
+        for k in (1, 2, 3, 64 // windows, 64 // windows + 1, 16384 // windows, 16384 // windows + 1):
+            idx = rng.integers(0, n, size=k).astype(np.uint64)
+            vals = oracle.uniform_fr(1500 + k, k)
+            assert backend.sparse_msm_resident(h, idx, vals, [0, k]) == [oracle.sparse_msm_g1(bases, idx, vals)], k
+    finally:
+        backend.release_bases(h)

@@ -1324,55 +1324,60 @@ void msm_run(MsmWorkspace& ws, const Affine<F>* d_points, const uint32_t* d_scal
 }
 
 // ---------------------------------------------------------------- direct small sparse MSMs
-constexpr int SD_BLOCK = 256;
+constexpr int SD_THREADS = 256, SD_TERMS = SD_THREADS / 4;
 struct SdJob {
     uint32_t request, first, items, pad;  // terms first .. first + items - 1 (term = entry W + window)
 };
 
-// XYZZ point read past L1: written by another block of this launch (made
+// Coordinate read past L1: written by another block of this launch (made
 // visible by its __threadfence before the counter increment below).
-DV_INL XYZZ<Fq> load_cg(const XYZZ<Fq>* p) {
-    XYZZ<Fq> r;
+DV_INL Fq load_cg(const Fq* p) {
+    Fq r;
     const uint4* src = reinterpret_cast<const uint4*>(p);
     uint4* dst = reinterpret_cast<uint4*>(&r);
-    for (int i = 0; i < (int)(sizeof(XYZZ<Fq>) / 16); ++i) dst[i] = __ldcg(src + i);
+    for (int i = 0; i < (int)(sizeof(Fq) / 16); ++i) dst[i] = __ldcg(src + i);
     return r;
 }
 
-// Tree sum of sm[0 .. live) into sm[0] (entries up to the next power of two
-// hold infinity): only the levels the live entries need.
-DV_INL void block_sum(XYZZ<Fq>* sm, uint32_t live) {
-    uint32_t span = 1;
-    while (span < live) span <<= 1;
-    for (uint32_t stride = span >> 1; stride > 0; stride >>= 1) {
-        if (threadIdx.x < (unsigned)stride)
-            sm[threadIdx.x] = XYZZ<Fq>::add_paired(sm[threadIdx.x], sm[threadIdx.x + stride]);
-        __syncthreads();
-    }
+// Sum over the block's quads; the first quad ends with it.
+DV_INL Fq quads_sum_block(Fq acc, Fq (*sh)[4]) {
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, r = threadIdx.x & 3;
+    acc = quads_sum_warp<Fq>(acc);
+    if (lane < 4) sh[warp][r] = acc;
+    __syncthreads();
+    if (warp == 0) acc = quads_sum_warp<Fq>(sh[lane >> 2][r]);
+    __syncthreads();
+    return acc;
 }
 
 // Sparse MSMs over a window table in one launch.  Each block takes up to
-// SD_BLOCK (entry, window) terms of one request: a thread forms d T (the
+// SD_TERMS (entry, window) terms of one request: a lane quad forms d T (the
 // signed c-bit digit d of the entry's window, T the table's multiple
-// 2^(c w) P) by double-and-add, the block sums its threads.  The last block
+// 2^(c w) P) by double-and-add, the block sums its quads.  The last block
 // of a request to finish (a per-request counter, reset by that block for the
 // next call) sums the request's block partials and writes the XYZZ sum.
+// The launch is one chain: up to c doublings and c / 2 additions, a tree of
+// six additions, the same over the partials, each three or four dependent
+// products in a quad.  256 entries of 32 windows, a whole call from host
+// memory: 210 us with a thread a term and one bit a step, 143 us so.
 // The host normalises all requests with one batch inversion, as the
 // reference does (icicle_msm.cu:417-421): one thread's inversion on the
 // device takes longer than that copy and a host batch inversion.
-__global__ void __launch_bounds__(SD_BLOCK) k_sparse_direct(const G1A* __restrict__ table, uint64_t nbases, int c,
+__global__ void __launch_bounds__(SD_THREADS) k_sparse_direct(const G1A* __restrict__ table, uint64_t nbases, int c,
                                                             int W, const uint64_t* __restrict__ idx,
                                                             const uint32_t* __restrict__ vals,
                                                             const SdJob* __restrict__ jobs,
                                                             const uint32_t* __restrict__ req_blocks,
                                                             XYZZ<Fq>* __restrict__ partial, uint32_t* __restrict__ done,
                                                             XYZZ<Fq>* __restrict__ out, uint32_t* __restrict__ err) {
-    __shared__ XYZZ<Fq> sm[SD_BLOCK];
+    __shared__ Fq sh[SD_THREADS / 32][4];
     __shared__ bool last;
     const SdJob job = jobs[blockIdx.x];
-    XYZZ<Fq> p = XYZZ<Fq>::inf();
-    if (threadIdx.x < job.items) {
-        const uint32_t term = job.first + threadIdx.x;
+    const uint32_t quad = threadIdx.x >> 2, r = threadIdx.x & 3;
+    uint32_t mag = 0;
+    Fq t = Quad<Fq>::inf();
+    if (quad < job.items) {
+        const uint32_t term = job.first + quad;
         const uint32_t e = term / (uint32_t)W, w = term % (uint32_t)W;
         uint32_t s[8];
         load_scalar(vals, e, s);
@@ -1387,39 +1392,41 @@ __global__ void __launch_bounds__(SD_BLOCK) k_sparse_direct(const G1A* __restric
             const uint32_t* words = vals + 8ull * e;
             const uint32_t d = window_raw(words, (int)w * c, c) + carry_into(words, (int)w, c);
             const bool neg = d > B;
-            const uint32_t mag = neg ? full - d : d;
-            const G1A t = table[ix * (uint64_t)W + w];
-            if (mag && !t.is_inf()) {
-                p = XYZZ<Fq>::from_affine(t);
-                for (int b = 30 - __clz(mag); b >= 0; --b) {
-                    p = XYZZ<Fq>::dbl_paired(p);
-                    if ((mag >> b) & 1) p = XYZZ<Fq>::add_affine(p, t);
-                }
-                if (neg) p = p.neg();
-            }
+            const G1A a = table[ix * (uint64_t)W + w];
+            mag = a.is_inf() ? 0u : neg ? full - d : d;
+            if (mag) t = r == 0 ? a.x : r == 1 ? (neg ? Fq::neg(a.y) : a.y) : Fq::one();
         }
     }
-    sm[threadIdx.x] = p;
-    __syncthreads();
-    block_sum(sm, job.items);
-    const uint32_t r = job.request, b0 = req_blocks[r], b1 = req_blocks[r + 1];
-    if (threadIdx.x == 0) {
-        partial[blockIdx.x] = sm[0];
-        __threadfence();
-        last = atomicAdd(done + r, 1u) == b1 - b0 - 1;
+    // d T by two bits a step over T, 2 T, 3 T, from each quad's top pair of
+    // bits on, the warp in step with its longest digit
+    const Fq t2 = Quad<Fq>::dbl(t), t3 = Quad<Fq>::add(t2, t);
+    const auto multiple = [&](uint32_t m) { return m == 1 ? t : m == 2 ? t2 : t3; };
+    const int top = mag ? (31 - __clz(mag)) >> 1 : -1;
+    Fq p = mag ? multiple(mag >> (2 * top)) : Quad<Fq>::inf();
+    for (int b = __reduce_max_sync(0xffffffffu, top) - 1; b >= 0; --b) {
+        const Fq four = Quad<Fq>::dbl(Quad<Fq>::dbl(p));
+        if (b < top) p = four;
+        const uint32_t m = b < top ? (mag >> (2 * b)) & 3u : 0u;
+        const Fq sum = Quad<Fq>::add(p, multiple(m));
+        if (m) p = sum;
     }
+    p = quads_sum_block(p, sh);
+    const uint32_t req = job.request, b0 = req_blocks[req], b1 = req_blocks[req + 1];
+    if (threadIdx.x < 4) {
+        reinterpret_cast<Fq*>(partial + blockIdx.x)[r] = p;
+        __threadfence();
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(done + req, 1u) == b1 - b0 - 1;
     __syncthreads();
     if (!last) return;
     __threadfence();
-    p = XYZZ<Fq>::inf();
-    for (uint32_t b = b0 + threadIdx.x; b < b1; b += SD_BLOCK) p = XYZZ<Fq>::add_paired(p, load_cg(partial + b));
-    sm[threadIdx.x] = p;
-    __syncthreads();
-    block_sum(sm, (b1 - b0) < (uint32_t)SD_BLOCK ? b1 - b0 : (uint32_t)SD_BLOCK);
-    if (threadIdx.x == 0) {
-        done[r] = 0;
-        out[r] = sm[0];
-    }
+    p = Quad<Fq>::inf();
+    for (uint32_t b = b0 + quad; __any_sync(0xffffffffu, b < b1); b += SD_TERMS)
+        p = Quad<Fq>::add(p, b < b1 ? load_cg(reinterpret_cast<const Fq*>(partial + b) + r) : Quad<Fq>::inf());
+    p = quads_sum_block(p, sh);
+    if (threadIdx.x < 4) reinterpret_cast<Fq*>(out + req)[r] = p;
+    if (threadIdx.x == 0) done[req] = 0;
 }
 
 void msm_sparse_direct(MsmWorkspace& ws, const MsmPrecomp<Fq>& pre, uint64_t nbases, const uint64_t* d_idx,
@@ -1431,8 +1438,8 @@ void msm_sparse_direct(MsmWorkspace& ws, const MsmPrecomp<Fq>& pre, uint64_t nba
     bool empty = false;
     for (uint32_t r = 0; r < count; ++r) {
         const uint32_t first = offs[r] * W, terms = (offs[r + 1] - offs[r]) * W;
-        for (uint32_t t = 0; t < terms; t += SD_BLOCK)
-            jobs.push_back(SdJob{r, first + t, std::min<uint32_t>(SD_BLOCK, terms - t), 0});
+        for (uint32_t t = 0; t < terms; t += SD_TERMS)
+            jobs.push_back(SdJob{r, first + t, std::min<uint32_t>(SD_TERMS, terms - t), 0});
         req_blocks[r + 1] = (uint32_t)jobs.size();
         empty |= terms == 0;
     }
@@ -1455,7 +1462,7 @@ void msm_sparse_direct(MsmWorkspace& ws, const MsmPrecomp<Fq>& pre, uint64_t nba
     DV_CUDA(cudaMemsetAsync(d_done, 0, count * sizeof(uint32_t), st));
     if (empty) DV_CUDA(cudaMemsetAsync(d_out, 0, (size_t)count * XB, st));  // all-zero XYZZ: infinity
     DV_CUDA(cudaMemsetAsync(d_err, 0xff, 2 * sizeof(uint32_t), st));
-    k_sparse_direct<<<(unsigned)jobs.size(), SD_BLOCK, 0, st>>>(
+    k_sparse_direct<<<(unsigned)jobs.size(), SD_THREADS, 0, st>>>(
         pre.table, nbases, pre.c, (int)W, d_idx, d_vals, reinterpret_cast<const SdJob*>(d_desc),
         reinterpret_cast<const uint32_t*>(d_desc + jb), d_partial, d_done, reinterpret_cast<XYZZ<Fq>*>(d_out), d_err);
     DV_LAUNCH();
