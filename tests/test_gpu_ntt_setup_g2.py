@@ -168,3 +168,20 @@ def test_random_twist_points_are_off_subgroup(backend, oracle):
         assert (expect == 4).all(), alg
         masks, rep = backend.inspect_g2_validation(wire, alg)
         assert (masks == expect).all() and rep.invalid_points == n, alg
+
+
+@pytest.mark.parametrize("algorithm", [1, 2, 3])
+@pytest.mark.parametrize("n", [1, 9, 4736, 4737])
+def test_g2_check_lane_layouts(backend, oracle, golden, algorithm, n):
+    """A lane quad a point up to 4736 points and a thread each beyond: the
+    golden wire corpus (flags, bad encodings, infinity) repeated among valid and
+    twist points, around both edges and in a ragged warp."""
+    wire = b"".join(H(w) for w in golden["g2_check"]["wire"]) + oracle.g2_twist_points(1720002, 7)
+    wire += oracle.fixed_base_g2(oracle.uniform_fr(1720003, 7))
+    count = len(wire) // 128
+    start = n % count  # another first point each time
+    order = [(start + i) % count for i in range(n)]
+    expect = oracle.g2_check(wire, algorithm).tolist()
+    masks, rep = backend.inspect_g2_validation(b"".join(wire[128 * i:128 * i + 128] for i in order), algorithm)
+    assert masks.tolist() == [expect[i] for i in order]
+    assert rep.checked_points == n and rep.invalid_points == sum(expect[i] != 0 for i in order)
