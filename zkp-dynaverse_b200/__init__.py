@@ -328,6 +328,19 @@ def _as_bytes(data):
     return bytes(data)
 
 
+_bytes_of_size = ctypes.pythonapi.PyBytes_FromStringAndSize
+_bytes_of_size.restype = ctypes.py_object
+_bytes_of_size.argtypes = [ctypes.c_void_p, ctypes.c_ssize_t]
+
+
+def _result(n: int) -> bytes:
+    """A new, unfilled bytes object of n bytes for one library call to write
+    its result into before it is handed on (a new bytes object may be filled
+    until then).  A ctypes buffer would be cleared first, then copied by .raw and
+    once more by a slice: most of the time of calls with megabytes of results."""
+    return _bytes_of_size(None, n) if n > 0 else b""
+
+
 def encode_fr(v: int) -> bytes:
     if not 0 <= v < R_MODULUS:
         raise ValueError("scalar out of range")
@@ -764,9 +777,9 @@ class DvgpuBackend:
         n = len(values) // FR_BYTES
         if n == 0 or n & (n - 1) or len(values) != n * FR_BYTES:
             raise ValueError(f"ntt size {n} is not a power of two")
-        out = ctypes.create_string_buffer(n * FR_BYTES)
+        out = _result(n * FR_BYTES)
         self._call("dvgpu_bn254_ntt_ex", _ptr(values), n, int(bool(inverse)), out)
-        return out.raw
+        return out
 
     def ntt_with_root(self, values: bytes, inverse: bool, root: bytes) -> bytes:
         """The reference ABI form with the explicit 2^20 root (icicle.rs:440-446)."""
@@ -779,22 +792,22 @@ class DvgpuBackend:
         n = len(values) // FR_BYTES
         if n == 0 or n & (n - 1):
             raise ValueError(f"ntt size {n} is not a power of two")
-        out = ctypes.create_string_buffer(n * FR_BYTES)
+        out = _result(n * FR_BYTES)
         self._call("dvgpu_bn254_ntt_ex", _ptr(values), n, NTT_COSET_INVERSE if inverse else NTT_COSET_FORWARD, out)
-        return out.raw
+        return out
 
     # ------------------------------------------------------------------ fixed base
     def fixed_base_g1(self, scalars: bytes) -> bytes:
         n = len(scalars) // FR_BYTES
-        out = ctypes.create_string_buffer(max(1, n) * G1_BYTES)
-        self._call("dvgpu_bn254_fixed_base", _ptr(scalars), n, 0, out)
-        return out.raw[:n * G1_BYTES]
+        out = _result(n * G1_BYTES)
+        self._call("dvgpu_bn254_fixed_base", _ptr(scalars), n, 0, out or None)
+        return out
 
     def fixed_base_g2(self, scalars: bytes) -> bytes:
         n = len(scalars) // FR_BYTES
-        out = ctypes.create_string_buffer(max(1, n) * G2_BYTES)
-        self._call("dvgpu_bn254_fixed_base", _ptr(scalars), n, 1, out)
-        return out.raw[:n * G2_BYTES]
+        out = _result(n * G2_BYTES)
+        self._call("dvgpu_bn254_fixed_base", _ptr(scalars), n, 1, out or None)
+        return out
 
     def setup_stats(self) -> SetupStats:
         s = SetupStats()
@@ -842,10 +855,10 @@ class DvgpuBackend:
 
     def fixed_base_g2_checked(self, scalars: bytes, algorithm: int):
         n = len(scalars) // FR_BYTES
-        out = ctypes.create_string_buffer(max(1, n) * G2_BYTES)
+        out = _result(max(1, n) * G2_BYTES)
         rep = G2ValidationReport()
         self._call("dvgpu_bn254_fixed_base_g2_checked", _ptr(scalars), n, algorithm, out, ctypes.byref(rep))
-        return out.raw[:n * G2_BYTES], rep
+        return (out if n else b""), rep
 
     # ------------------------------------------------------------------ device forms
     def msm_device(self, d_points: int, d_scalars: int, n: int, g2=False, stream=None) -> bytes:
@@ -909,9 +922,9 @@ class DvgpuBackend:
         if row_len <= 0 or len(points) % (G1_BYTES * row_len):
             raise ValueError("points must hold whole rows")
         rows = len(points) // (G1_BYTES * row_len)
-        out = ctypes.create_string_buffer(max(1, len(points)))
+        out = _result(max(1, len(points)))
         self._call("dvgpu_bn254_g1_ntt_rows", _ptr(points), row_len, rows, int(inverse), out)
-        return out.raw[:len(points)]
+        return out if points else b""
 
     def g1_ntt_rows_device(self, d_points: int, row_len: int, rows: int, inverse: bool, d_out: int, stream=None):
         self._call("dvgpu_bn254_g1_ntt_rows_device", d_points, row_len, rows, int(inverse), d_out, stream)
@@ -950,9 +963,9 @@ class DvgpuBackend:
     def pairing(self, g1: bytes, g2: bytes) -> bytes:
         """e(P_i, Q_i): 384-byte GT elements (tower order, canonical)."""
         n = len(g1) // G1_BYTES
-        out = ctypes.create_string_buffer(max(1, 384 * n))
+        out = _result(max(1, 384 * n))
         self._call("dvgpu_bn254_pairing", g1, g2, n, out)
-        return out.raw[:384 * n]
+        return out if n else b""
 
     # ------------------------------------------------------------------ polynomial toolkit
     # crates/protocol/src/domain/fast.rs over canonical Fr coefficient bytes
@@ -1100,10 +1113,10 @@ class DvgpuBackend:
         forward)."""
         logs = np.ascontiguousarray(np.asarray(log_sizes, dtype=np.uint32))
         kd = None if kinds is None else np.ascontiguousarray(np.asarray(kinds, dtype=np.int32))
-        out = ctypes.create_string_buffer(max(1, len(values)))
+        out = _result(max(1, len(values)))
         self._call("dvgpu_bn254_ntt_batch", _ptr(values), logs.ctypes.data if logs.size else None,
                    None if kd is None else kd.ctypes.data, len(logs), out)
-        return out.raw[:len(values)]
+        return out if len(values) else b""
 
     def ntt_batch_device(self, d_values: int, log_sizes, d_out: int, kinds=None, stream=None):
         logs = np.ascontiguousarray(np.asarray(log_sizes, dtype=np.uint32))
@@ -1141,10 +1154,10 @@ class DvgpuBackend:
         results, concatenated NTT outputs)."""
         msm_out = ctypes.create_string_buffer(max(1, msm_count) * G1_BYTES)
         nbytes = 0 if ntt_values is None else len(ntt_values)
-        ntt_out = ctypes.create_string_buffer(max(1, nbytes))
+        ntt_out = _result(max(1, nbytes))
         self._call("dvgpu_batch_plan_run", plan, _ptr(scalars), _ptr(ntt_values), msm_out, ntt_out)
         raw = msm_out.raw
-        return [raw[i * G1_BYTES:(i + 1) * G1_BYTES] for i in range(msm_count)], ntt_out.raw[:nbytes]
+        return [raw[i * G1_BYTES:(i + 1) * G1_BYTES] for i in range(msm_count)], (ntt_out if nbytes else b"")
 
     def batch_plan_destroy(self, plan: int):
         self._call("dvgpu_batch_plan_destroy", plan)
