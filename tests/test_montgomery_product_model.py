@@ -159,3 +159,15 @@ def test_reduction_of_differences(p):
     for t in edge + [rng.randrange(-2 * (p - 1) ** 2, 2 * (p - 1) ** 2) for _ in range(1500)]:
         w = make_positive(_limbs(t % (1 << 512), 16), p)
         assert f.redc(w) == t * r_inv % p
+
+
+@pytest.mark.parametrize("p", [Q, R])
+def test_product_of_unreduced_operand(p):
+    """Fp::mul_lazy: a < p times b < 4p stays below 2p before the last
+    subtraction (asserted in finish) without losing a carry."""
+    f, rng, r_inv = Field(p), random.Random(9), pow(1 << 256, -1, p)
+    edge_b = [0, 1, p, 2 * p - 1, 2 * p, 3 * p, 4 * p - 1, 4 * p - 2]
+    cases = [(x, y) for x in (0, 1, p - 1, p - 2) for y in edge_b]
+    cases += [(rng.randrange(p), rng.randrange(4 * p)) for _ in range(1500)] + [(p - 1, rng.randrange(3 * p, 4 * p)) for _ in range(300)]
+    for x, y in cases:
+        assert f.mul(_limbs(x), _limbs(y)) == x * y * r_inv % p

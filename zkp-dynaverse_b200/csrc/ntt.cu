@@ -161,6 +161,7 @@ DV_INL void dif_round(const PassArgs& a, uint32_t* sm, int tile_log, uint64_t fi
     const uint32_t TE = 1u << tile_log;
     const int b_lo = bit_hi - RR;
     const bool last_round = b_lo == 0;
+    const bool ends = last_round && lb == 0;
     const uint32_t lanes = TE >> RR;
     for (uint32_t tau = threadIdx.x; tau < lanes; tau += THREADS) {
         const uint32_t base_t = ((tau >> b_lo) << bit_hi) | (tau & ((1u << b_lo) - 1));
@@ -183,8 +184,8 @@ DV_INL void dif_round(const PassArgs& a, uint32_t* sm, int tile_log, uint64_t fi
                     }
 #pragma unroll
                     for (int j = 0; j < 8; ++j) x[m].v[j] = c[j];
-                    // values stay canonical: multipliers are held in
-                    // Montgomery form and mont_mul(a, x R) = a x
+                    // values stay out of Montgomery form: multipliers are in
+                    // it and mont_mul(a, x R) = a x
                     if (a.pre_hi) {
                         const uint64_t lo_mask = (1ull << a.split) - 1;
                         x[m] = Fr::mul_inl(Fr::mul_inl(x[m], a.pre_hi[idx >> a.split]), a.pre_lo[idx & lo_mask]);
@@ -201,21 +202,27 @@ DV_INL void dif_round(const PassArgs& a, uint32_t* sm, int tile_log, uint64_t fi
             const int s = a.s0 + (k - bit_hi) + j;  // global stage
             const int pb = bit_hi - 1 - j;          // local bit of this stage
             const int hs = 1 << (RR - 1 - j);      // pair distance in m
-            // issue this stage's twiddle loads before its butterflies
+            // issue this stage's twiddle loads before its butterflies; in the
+            // transform's last round pairs with no element bit below the
+            // stage's have the twiddle 1
             Fr w[R / 2];
 #pragma unroll
             for (int m = 0, q = 0; m < R; ++m) {
                 if (m & hs) continue;
                 const uint32_t e = base_e | ((uint32_t)m << b_lo);
                 const uint64_t jp = ((uint64_t)(e & ((1u << pb) - 1)) << lb) | low;
-                w[q++] = a.tw[jp << s];
+                if ((m & (hs - 1)) || !ends) w[q] = a.tw[jp << s];
+                ++q;
             }
+            // values between the stages are below 2r, differences below 4r
 #pragma unroll
             for (int m = 0, q = 0; m < R; ++m) {
                 if (m & hs) continue;
-                const Fr u = x[m], v = x[m + hs];
-                x[m] = Fr::add(u, v);
-                x[m + hs] = Fr::mul_inl(Fr::sub(u, v), w[q++]);
+                const Fr u = x[m], d = Fr::sub_2p(u, x[m + hs]);
+                x[m] = Fr::reduce_2p(Fr::add_raw(u, x[m + hs]));
+                if ((m & (hs - 1)) || !ends) x[m + hs] = Fr::mul_lazy(w[q], d);
+                else x[m + hs] = Fr::reduce_2p(d);
+                ++q;
             }
         }
 #pragma unroll
@@ -231,6 +238,8 @@ DV_INL void dif_round(const PassArgs& a, uint32_t* sm, int tile_log, uint64_t fi
                         y = Fr::mul_inl(Fr::mul_inl(y, a.post_hi[i >> a.split]), a.post_lo[i & lo_mask]);
                     } else if (a.post_const) {
                         y = Fr::mul_inl(y, *a.post_const);
+                    } else {
+                        Fr::reduce_once(y.v);
                     }
                     store_words(a.out + 32 * i, y.v);
                 } else {
@@ -264,8 +273,13 @@ DV_INL void dif_tile(const PassArgs& a, uint32_t* sm, int tile_log, uint64_t fir
 #ifndef DV_NTT_MINB
 #define DV_NTT_MINB 3
 #endif
+// Radix-2 rounds: one product a lane and round, 78 registers and no spills at
+// three blocks an SM.  2^22 with the inverse coset scaling 1.00 ms, radix 4
+// 1.01 (two blocks 1.02), radix 8 1.11; 2^12, where a round is the latency of its
+// products, 31.7, 37.8 and 56 us.  Loading a twiddle one butterfly ahead took
+// 1.06 ms: the registers cost more than the wait.
 #ifndef DV_NTT_RADIX_LOG
-#define DV_NTT_RADIX_LOG 2
+#define DV_NTT_RADIX_LOG 1
 #endif
 template <int THREADS, int R_LOG>
 __global__ void __launch_bounds__(THREADS, (THREADS >= 256 ? DV_NTT_MINB : 8)) k_dif_pass(const PassArgs a) {
@@ -296,7 +310,7 @@ __global__ void __launch_bounds__(THREADS, (THREADS >= 256 ? DV_NTT_MINB : 8)) k
     }
 }
 
-// Bit-reversal permutation + post scaling (values are already canonical).
+// Bit-reversal permutation + post scaling (values below 2r made canonical).
 __global__ void k_permute(const Fr* __restrict__ work, uint8_t* __restrict__ out, int logn,
                           const Fr* __restrict__ post_hi, const Fr* __restrict__ post_lo, int split,
                           const Fr* __restrict__ post_const) {
@@ -309,6 +323,8 @@ __global__ void k_permute(const Fr* __restrict__ work, uint8_t* __restrict__ out
         a = Fr::mul_inl(Fr::mul_inl(a, post_hi[i >> split]), post_lo[i & lo_mask]);
     } else if (post_const) {
         a = Fr::mul_inl(a, *post_const);
+    } else {
+        Fr::reduce_once(a.v);
     }
     store_words(out + 32 * i, a.v);
 }
@@ -436,8 +452,12 @@ void ntt_run(NttWorkspace& ws, const uint8_t* d_in, uint8_t* d_out, int logn, in
     const uint64_t n = 1ull << logn;
     const Scaling sc = scaling_of(tab, kind);
     Fr* work = ws.work.as<Fr>(n);
+    // the error word stays at "none" from call to call, so only a call that
+    // follows a bad input (or the first) sets it
     uint32_t* bad = ws.err.as<uint32_t>(1);
-    DV_CUDA(cudaMemsetAsync(bad, 0xff, sizeof(uint32_t), st));
+    uint32_t* host_bad = ws.host_err.as<uint32_t>(1);
+    if (!ws.err_clear) DV_CUDA(cudaMemsetAsync(bad, 0xff, sizeof(uint32_t), st));
+    ws.err_clear = false;
 
     if (!run_passes(d_in, work, d_out, logn, sc.tw, sc.pre_hi, sc.pre_lo, sc.post_hi, sc.post_lo, sc.post_const,
                     sc.split, bad, true, st)) {
@@ -445,10 +465,11 @@ void ntt_run(NttWorkspace& ws, const uint8_t* d_in, uint8_t* d_out, int logn, in
                                                               sc.post_const);
         DV_LAUNCH();
     }
-    uint32_t host_bad = 0;
-    DV_CUDA(cudaMemcpyAsync(&host_bad, bad, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+    DV_CUDA(cudaMemcpyAsync(host_bad, bad, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
     DV_CUDA(cudaStreamSynchronize(st));
-    if (host_bad != 0xffffffffu) throw InvalidArgument("non-canonical NTT input at index " + std::to_string(host_bad));
+    if (*host_bad != 0xffffffffu)
+        throw InvalidArgument("non-canonical NTT input at index " + std::to_string(*host_bad));
+    ws.err_clear = true;
     ws.calls++;
     ws.elements += n;
 }

@@ -10,14 +10,15 @@
 // before the transform, inverse scales output i by g^-i after it.
 //
 // Layout: canonical little-endian 32-byte elements in HBM (the wire format).
-// Values stay canonical throughout: every multiplier (twiddles, coset and
-// scale factors) is held in Montgomery form, and mont_mul(a, x R) = a x.
+// Values stay out of Montgomery form: every multiplier (twiddles, coset and
+// scale factors) is held in it, and mont_mul(a, x R) = a x.  Between the
+// stages they are only kept below 2r; the output is canonical.
 // The transform is decimation-in-frequency radix-2, grouped into passes of
 // up to 11 stages; each pass stages a tile of 2^11 elements (one group of
 // 2^k elements with stride 2^lb, or several consecutive groups when k < 11)
 // in shared memory as two swizzled planes of 16-byte halves and runs its
-// stages in register rounds of two (each thread owns 4 elements per round),
-// with twiddles from a resident table w^i (i < n/2).  The last pass writes
+// stages in register rounds (each thread owns 2 elements per round, 4 or 8 in
+// batches that ask for it), with twiddles from a resident table w^i (i < n/2).  The last pass writes
 // the output in natural order (bit reversal fused with the inverse and
 // coset scaling).
 //
@@ -51,6 +52,8 @@ struct NttTables {
 struct NttWorkspace {
     DevBuf work;
     DevBuf err;
+    PinnedBuf host_err;
+    bool err_clear = false;  // err holds "none"
     std::map<int, std::unique_ptr<NttTables>> tables;  // key: logn * 4 + kind
     uint64_t calls = 0, elements = 0;
 };
