@@ -617,7 +617,28 @@ __global__ void k_dv_geom(FieldCtx c) {
 // the points come from the table of w^k), one warp per point with the
 // product split over its lanes, then an inverse transform of size N in
 // shared memory.  The chain is about a / 32 + log N + 5 products, against a
-// for the product taken one factor at a time.
+// for the product taken one factor at a time.  The N values are a N products,
+// too many for one SM once a is in the tens (a = 100: 128 us in this kernel,
+// 31 us for both): k_dv_vanish_values then spreads them over the GPU, a
+// warp a value, into the job's matrix scratch (a a elements, unused yet).
+constexpr uint32_t VANISH_SPLIT = 16;  // affected points up to which one block does it all
+DV_INL Fr vanish_value(const Fr& y, const Fr* x, uint32_t a, uint32_t lane) {
+    Fr p = Fr::one();
+    for (uint32_t k = lane; k < a; k += 32) p = Fr::mul(p, Fr::sub(y, x[k]));
+    for (int m = 16; m >= 1; m >>= 1) p = Fr::mul(p, shfl_xor_fr(p, m));
+    return p;
+}
+__global__ void __launch_bounds__(256) k_dv_vanish_values(FieldCtx c) {
+    const FieldJob J = c.jobs[blockIdx.y];
+    const uint32_t a = J.a, lane = threadIdx.x & 31;
+    if (a <= VANISH_SPLIT) return;
+    const uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    uint32_t logN = 0;
+    while ((1u << logN) < a + 1) ++logN;
+    if (i >> logN) return;
+    const Fr p = vanish_value(c.wpow[(i * (c.n >> logN)) & (c.n - 1)], c.scr + J.scr + s_X(a), a, lane);
+    if (lane == 0) c.scr[J.mat + i] = p;
+}
 __global__ void __launch_bounds__(1024) k_dv_vanish(FieldCtx c) {
     extern __shared__ Fr sm[];
     const uint32_t jb = blockIdx.x;
@@ -629,12 +650,13 @@ __global__ void __launch_bounds__(1024) k_dv_vanish(FieldCtx c) {
     while ((1u << logN) < a + 1) ++logN;
     const uint32_t N = 1u << logN, step = c.n >> logN, mask = c.n - 1;
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarp = blockDim.x >> 5;
-    for (uint32_t i = warp; i < N; i += nwarp) {
-        const Fr y = c.wpow[(i * step) & mask];
-        Fr p = Fr::one();
-        for (uint32_t k = lane; k < a; k += 32) p = Fr::mul(p, Fr::sub(y, s[s_X(a) + k]));
-        for (int m = 16; m >= 1; m >>= 1) p = Fr::mul(p, shfl_xor_fr(p, m));
-        if (lane == 0) sm[logN ? __brev(i) >> (32 - logN) : 0] = p;
+    if (a > VANISH_SPLIT) {
+        for (uint32_t i = threadIdx.x; i < N; i += blockDim.x) sm[__brev(i) >> (32 - logN)] = c.scr[J.mat + i];
+    } else {
+        for (uint32_t i = warp; i < N; i += nwarp) {
+            const Fr p = vanish_value(c.wpow[(i * step) & mask], s + s_X(a), a, lane);
+            if (lane == 0) sm[logN ? __brev(i) >> (32 - logN) : 0] = p;
+        }
     }
     __syncthreads();
     // inverse transform (decimation in time, bit-reversed input)
@@ -2427,6 +2449,10 @@ void Engine::run_sparse(Params& P, std::vector<Job*>& jobs) {
     }
     uint64_t vanish_n = 1;  // the largest transform of k_dv_vanish
     while (vanish_n < amax + 1) vanish_n <<= 1;
+    if (amax > VANISH_SPLIT) {
+        k_dv_vanish_values<<<dim3((unsigned)((vanish_n + 7) / 8), B), 256, 0, st>>>(c);
+        DV_LAUNCH();
+    }
     k_dv_vanish<<<B, 1024, vanish_n * sizeof(Fr), st>>>(c);
     DV_LAUNCH();
     if (K) {
