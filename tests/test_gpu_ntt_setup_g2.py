@@ -185,3 +185,22 @@ def test_g2_check_lane_layouts(backend, oracle, golden, algorithm, n):
     masks, rep = backend.inspect_g2_validation(b"".join(wire[128 * i:128 * i + 128] for i in order), algorithm)
     assert masks.tolist() == [expect[i] for i in order]
     assert rep.checked_points == n and rep.invalid_points == sum(expect[i] != 0 for i in order)
+
+
+@pytest.mark.parametrize("logn", [6, 7, 8, 9, 10, 11, 12, 15, 16, 17])
+@pytest.mark.parametrize("kind", [0, 1, 2, 3])
+def test_ntt_pass_and_block_edges(backend, oracle, logn, kind):
+    """One and two passes (2^9, 2^10), tiles of 2^6 to 2^9 elements with their
+    block sizes, values at both ends of the field, in place and not."""
+    import torch
+    n = 1 << logn
+    r = 0x30644E72E131A029B85045B68181585D2833E84879B9709143E1F593F0000001
+    vals = (r - 1).to_bytes(32, "little") * 3 + bytes(64) + oracle.uniform_fr(7300 + logn, n - 5)
+    expect = oracle.ntt(vals, ["forward", "inverse", "coset_forward", "coset_inverse"][kind])
+    d = torch.frombuffer(bytearray(vals), dtype=torch.uint8).cuda()
+    out = torch.empty_like(d)
+    torch.cuda.synchronize()
+    backend.ntt_device(d.data_ptr(), n, kind, out.data_ptr())
+    assert out.cpu().numpy().tobytes() == expect
+    backend.ntt_device(d.data_ptr(), n, kind, d.data_ptr())
+    assert d.cpu().numpy().tobytes() == expect
