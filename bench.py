@@ -250,7 +250,7 @@ class MsmOp:
         adds = tl.accum_mixed_adds / max(1, tl.calls)
         macs = adds * (G2_MADD_MACS if self.g2 else G1_MADD_MACS)
         ach = macs / (accum_ms * 1e-3) / 1e12
-        return ({"bound": "imad", "kernel": "k_accum (bucket accumulation)", "achieved": ach,
+        return ({"bound": "imad", "kernel": "bucket accumulation (k_accum, for long G1 lists behind k_pair_level), every addition counted as a mixed one", "achieved": ach,
                  "peak": imad_peak / 1e12, "unit": "TMAC/s", "frac": ach / (imad_peak / 1e12),
                  "algorithmic_macs_per_launch": macs, "launch_ms": accum_ms},
                 {"algorithmic_macs": macs_total, "achieved_tmacs": macs_total / (step_ms * 1e-3) / 1e12,
@@ -1188,7 +1188,7 @@ class ProofServeOp:
                                     "p99_ratio": poi_plain["p99_ms"] / poi_served["p99_ms"]},
                         "bit_exact": exact, "device_verifier_sample_accepted": bool(sample_ok)},
             "roofline": {"bound": "imad",
-                         "kernel": "k_accum of the dense MSMs (anchor openings, re-anchor quotients; c = 16 table)",
+                         "kernel": "k_pair_level and k_accum of the dense MSMs (anchor openings, re-anchor quotients; c = 16 table), every addition counted as a mixed one",
                          "achieved": acc_ach, "peak": peak, "unit": "TMAC/s", "frac": acc_ach / peak,
                          "peak_source": "dvgpu_probe_imad_rate, measured in this run",
                          "algorithmic_macs_per_launch": acc_macs / max(1, sat_served["batches"]),
@@ -1557,34 +1557,32 @@ def poly_cpu(oracle, points, values9, weighted3):
 
 
 def pairing_fme(equations, terms_per_eq, distinct_g2, per_equation):
-    """Fq multiplications of the lane-group pairing as implemented, all six
-    lanes of a group counted: an Fq12 product is a three-term Karatsuba over
-    Fq4, 18 Fq2 products (54 Fq-mul); a square the same with Fq4 squares, 18
-    Fq2 squares (36); a cyclotomic square 12 Fq2 squares (24); a sparse line
-    product 18 Fq2 products (54); the product of two lines 6 Fq2 products
-    (18); scaling a line by its P 4 Fq-mul.  Each distinct G2 point is
-    prepared once: 65 doublings and 23 additions whose Fq2 products are
-    spread over the group (13 and 16 per step, 3 Fq-mul each).  The Miller
-    loops, 65 squares and 88 line steps: one per term (per_equation false;
-    the terms' values then meet in one product each), or the multi-Miller
-    loop of two-term equations (per_equation true: one square per step, both
-    lines scaled, multiplied together and into f by one product).  Per
-    equation: the easy part (an Fq6 inverse, counted once although every
-    lane of the group repeats it: 37 Fq-mul and an Fq inverse by divsteps,
-    integer work counted as its one closing Montgomery product; four
-    products, two of them inside the inverse, and a q^2 Frobenius); three
-    exponentiations by z over its width-4 NAF
-    (63 cyclotomic squares and 16 products each); and the hard part's 13
-    products, 8 cyclotomic squares and three Frobenius maps
-    (18 + 12 + 30)."""
-    prep = 65 * 13 * 3 + 23 * 16 * 3
+    """Multiply-adds of the lane-group pairing as implemented, in Fq products
+    of MAC_MUL each, all twelve working lanes of a group counted.  A lane sums
+    the base products of its component (64 multiply-adds each) and reduces once
+    (72): an Fq12 product is 12 base products a lane, a square 8, a sparse line
+    product 6, a cyclotomic square 3; scaling a line by its P is 4 Fq products.
+    Each distinct G2 point is prepared once: 65 doublings and 23 additions of
+    11 and 13 Fq2 products, two lanes of two base products each.  The Miller
+    loops, 64 squares and 88 line steps: one per term (per_equation false; the
+    terms' values then meet in one product each), or one per two-term equation
+    (per_equation true).  Per equation: the easy part (an Fq6 inverse, counted
+    once although every lane of the group repeats it: 37 Fq products and an
+    Fq inverse by divsteps, integer work counted as its one closing Montgomery
+    product; four products, two of them inside the inverse, and a q^2
+    Frobenius); three exponentiations by z over its width-4 NAF (63 cyclotomic
+    squares and 16 products each); and the hard part's 13 products, 8
+    cyclotomic squares and three Frobenius maps (18 + 12 + 30)."""
+    dot = lambda products: 12 * (64 * products + 72) / MAC_MUL
+    full, square, line, cyclotomic = dot(12), dot(8), dot(6), dot(3)
+    prep = (65 * 11 + 23 * 13) * 2 * (2 * 64 + 72) / MAC_MUL
     if per_equation:
         assert terms_per_eq == 2
-        miller = 65 * 36 + 88 * (8 + 18 + 54)
+        miller = 64 * square + 88 * 2 * (4 + line)
     else:
-        miller = terms_per_eq * (65 * 36 + 88 * (4 + 54)) + (terms_per_eq - 1) * 54
-    easy = (37 + 1) + 4 * 54 + 12
-    hard = 3 * (63 * 24 + 16 * 54) + 13 * 54 + 8 * 24 + (18 + 12 + 30)
+        miller = terms_per_eq * (64 * square + 88 * (4 + line)) + (terms_per_eq - 1) * full
+    easy = (37 + 1) + 4 * full + 12
+    hard = 3 * (63 * cyclotomic + 16 * full) + 13 * full + 8 * cyclotomic + (18 + 12 + 30)
     return distinct_g2 * prep + equations * (miller + easy + hard)
 
 
@@ -1645,9 +1643,9 @@ class PairingOp:
 
     def per_equation(self, torch):
         """Whether the library runs the multi-Miller loop for this batch: more
-        terms than one wave of per-term groups (k_miller_multi at 206
-        registers holds 2 blocks of 20 groups per SM)."""
-        return 2 * self.eqs > torch.cuda.get_device_properties(0).multi_processor_count * 2 * 20
+        terms than one wave of per-term groups (k_miller_multi at 96
+        registers holds 5 blocks of 8 groups per SM)."""
+        return 2 * self.eqs > torch.cuda.get_device_properties(0).multi_processor_count * 5 * 8
 
     def roofline(self, tl, imad_peak, step_ms):
         import torch

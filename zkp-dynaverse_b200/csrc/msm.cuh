@@ -92,7 +92,7 @@ struct MsmPrecomp {
 // count canonical affine points (2 * sizeof(F) bytes each, all-zero for
 // infinity).  Throws InvalidArgument for non-canonical scalars.
 // Sparse MSMs over a resident table of window multiples, summed directly:
-// each (entry, window) term d T is formed by one thread (double-and-add on
+// each (entry, window) term d T is formed by four lanes (double-and-add on
 // the signed c-bit digit d), then block and request sums.  For small
 // supports, where the bucket pipeline's launch chain dominates.  d_idx:
 // entry base indices (checked < nbases), d_vals: canonical scalars (checked),
