@@ -204,3 +204,30 @@ def test_ntt_pass_and_block_edges(backend, oracle, logn, kind):
     assert out.cpu().numpy().tobytes() == expect
     backend.ntt_device(d.data_ptr(), n, kind, d.data_ptr())
     assert d.cpu().numpy().tobytes() == expect
+
+
+@pytest.mark.parametrize("logn", [0, 1, 9, 10, 11, 17])
+def test_ntt_reports_the_first_bad_value_and_recovers(backend, oracle, logn):
+    """The error word reaches the host from the last pass: one element, one
+    block, two passes; several bad values, then good calls again."""
+    import torch
+    n = 1 << logn
+    r = (0x30644E72E131A029B85045B68181585D2833E84879B9709143E1F593F0000001).to_bytes(32, "little")
+    good = oracle.uniform_fr(7400 + logn, n)
+    expect = oracle.ntt(good, "forward")
+
+    def on_device(data):
+        d = torch.frombuffer(bytearray(data), dtype=torch.uint8).cuda()
+        out = torch.empty_like(d)
+        torch.cuda.synchronize()
+        backend.ntt_device(d.data_ptr(), n, 0, out.data_ptr())
+        return out.cpu().numpy().tobytes()
+
+    assert on_device(good) == expect
+    for first in sorted({n - 1, n // 2, 0}):
+        bad = bytearray(good)
+        for at in {first, n - 1}:
+            bad[32 * at:32 * at + 32] = r
+        with pytest.raises(Exception, match=rf"index {first}\b"):
+            on_device(bytes(bad))
+        assert on_device(good) == expect

@@ -122,6 +122,7 @@ struct PassArgs {
     const Fr* post_const;     // fused last pass: n^-1 (plain inverse)
     uint32_t* first_bad;      // lowest non-canonical input index
     int logn, s0, k, first, split;
+    uint32_t* host_bad;       // last pass of a call that waits: first_bad's copy in pinned memory, or null
 };
 
 // One DIF pass over stages [s0, s0 + k) for one group of G = 2^k elements
@@ -308,6 +309,10 @@ __global__ void __launch_bounds__(THREADS, (THREADS >= 256 ? DV_NTT_MINB : THREA
             a.work[idx] = v;
         }
     }
+    // every check is in an earlier pass or, with one pass, in this one block
+    // before its last barrier
+    if (a.host_bad && blockIdx.x == 0 && threadIdx.x == 0)
+        *a.host_bad = *static_cast<volatile const uint32_t*>(a.first_bad);
 }
 
 // Bit-reversal permutation + post scaling (values below 2r made canonical).
@@ -358,9 +363,10 @@ void launch_pass(const PassArgs& a, cudaStream_t st) {
 // (otherwise k_permute must run).
 bool run_passes(const uint8_t* d_in, Fr* work, uint8_t* d_out, int logn, const Fr* tw, const Fr* pre_hi,
                 const Fr* pre_lo, const Fr* post_hi, const Fr* post_lo, const Fr* post_const, int split,
-                uint32_t* bad, bool fuse_out, cudaStream_t st) {
-    PassArgs a{d_in, work, nullptr, tw, pre_hi, pre_lo, post_hi, post_lo, post_const, bad, logn, 0, 0, 1, split};
+                uint32_t* bad, uint32_t* host_bad, bool fuse_out, cudaStream_t st) {
+    PassArgs a{d_in, work, nullptr, tw, pre_hi, pre_lo, post_hi, post_lo, post_const, bad, logn, 0, 0, 1, split, nullptr};
     if (logn == 0) {
+        a.host_bad = host_bad;
         // single element: conversion round trip checks canonical form
         launch_pass<32>(a, st);
         return false;
@@ -375,6 +381,7 @@ bool run_passes(const uint8_t* d_in, Fr* work, uint8_t* d_out, int logn, const F
         a.s0 = s0;
         a.first = p == 0;
         a.out = (fused && p == passes - 1) ? d_out : nullptr;
+        a.host_bad = p == passes - 1 ? host_bad : nullptr;
         // a thread a butterfly up to 2^9 elements a tile (2^15: 34 us, 43 with 64
         // threads on 2^8 elements; 2^8: 30 and 34)
         if (a.k >= 9) launch_pass<256>(a, st);
@@ -459,19 +466,19 @@ void ntt_run(NttWorkspace& ws, const uint8_t* d_in, uint8_t* d_out, int logn, in
     const Scaling sc = scaling_of(tab, kind);
     Fr* work = ws.work.as<Fr>(n);
     // the error word stays at "none" from call to call, so only a call that
-    // follows a bad input (or the first) sets it
+    // follows a bad input (or the first) sets it; the last pass writes it to
+    // the host
     uint32_t* bad = ws.err.as<uint32_t>(1);
     uint32_t* host_bad = ws.host_err.as<uint32_t>(1);
     if (!ws.err_clear) DV_CUDA(cudaMemsetAsync(bad, 0xff, sizeof(uint32_t), st));
     ws.err_clear = false;
 
     if (!run_passes(d_in, work, d_out, logn, sc.tw, sc.pre_hi, sc.pre_lo, sc.post_hi, sc.post_lo, sc.post_const,
-                    sc.split, bad, true, st)) {
+                    sc.split, bad, host_bad, true, st)) {
         k_permute<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(work, d_out, logn, sc.post_hi, sc.post_lo, sc.split,
                                                               sc.post_const);
         DV_LAUNCH();
     }
-    DV_CUDA(cudaMemcpyAsync(host_bad, bad, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
     DV_CUDA(cudaStreamSynchronize(st));
     if (*host_bad != 0xffffffffu)
         throw InvalidArgument("non-canonical NTT input at index " + std::to_string(*host_bad));
@@ -758,7 +765,7 @@ void ntt_noalloc(const uint8_t* d_in, uint8_t* d_out, int logn, int kind, cudaSt
     }
     const Fr* pre_hi = (coset && !inverse) ? hi : nullptr;
     const Fr* pre_lo = (coset && !inverse) ? lo : nullptr;
-    run_passes(d_in, work, d_out, logn, tw, pre_hi, pre_lo, nullptr, nullptr, nullptr, split, bad, false, st);
+    run_passes(d_in, work, d_out, logn, tw, pre_hi, pre_lo, nullptr, nullptr, nullptr, split, bad, nullptr, false, st);
     k_permute<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(work, d_out, logn, (coset && inverse) ? hi : nullptr,
                                                           (coset && inverse) ? lo : nullptr, split,
                                                           inverse ? kc + C_NINV : nullptr);
