@@ -397,3 +397,27 @@ def test_sparse_direct_block_edges(backend, oracle, c):
             assert backend.sparse_msm_resident(h, idx, vals, [0, k]) == [oracle.sparse_msm_g1(bases, idx, vals)], k
     finally:
         backend.release_bases(h)
+
+
+@pytest.mark.parametrize("n", [1, 300, 5000])
+@pytest.mark.parametrize("g2", [False, True])
+def test_msm_error_words_reach_the_host(dv, backend, oracle, n, g2):
+    """The last reduction kernel leaves the sums and both error words in host
+    memory: a bad point, a bad scalar, both (the scalar is named), and good
+    calls in between."""
+    size = 128 if g2 else 64
+    call = backend.msm_g2_host if g2 else backend.msm
+    pts, scs = _case_inputs(oracle, 8100 + n, n, g2)
+    expect = (oracle.msm_g2 if g2 else oracle.msm_g1)(pts, scs)
+    r = (0x30644E72E131A029B85045B68181585D2833E84879B9709143E1F593F0000001).to_bytes(32, "little")
+    assert call(pts, scs) == expect
+    for at in sorted({0, n - 1}):
+        bad_pts = pts[:at * size] + b"\x01" + bytes(size - 1) + pts[(at + 1) * size:]
+        bad_scs = scs[:32 * at] + r + scs[32 * at + 32:]
+        for p, s, message in ((bad_pts, scs, f"invalid point at index {at}"),
+                              (pts, bad_scs, f"non-canonical scalar at index {at}"),
+                              (bad_pts, bad_scs, f"non-canonical scalar at index {at}")):
+            with pytest.raises(dv.DvgpuError) as e:
+                call(p, s)
+            assert e.value.status == -1 and message in e.value.message
+            assert call(pts, scs) == expect

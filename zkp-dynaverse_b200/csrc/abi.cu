@@ -76,9 +76,9 @@ void msm_sets_device(Backend& b, const uint8_t* d_points, const uint8_t* d_scala
     uint32_t* bad = b.err.as<uint32_t>(1);
     DV_CUDA(cudaMemsetAsync(bad, 0xff, sizeof(uint32_t), st));
     convert_points<F>(d_points, conv, n, bad, st);
+    uint32_t first_bad = 0xffffffffu;
     msm_run<F>(b.msm, conv, reinterpret_cast<const uint32_t*>(d_scalars), offs.data(), count, window_for<F>(b, offs),
-               st, tmp.data(), &b.msm_stats);
-    const uint32_t first_bad = read_err_word(b, bad, st);
+               st, tmp.data(), &b.msm_stats, nullptr, bad, &first_bad);
     if (first_bad != 0xffffffffu) throw InvalidArgument("invalid point at index " + std::to_string(first_bad));
     memcpy(result, tmp.data(), tmp.size());
 }

@@ -814,7 +814,8 @@ __global__ void __launch_bounds__(128) k_segments(const XYZZ<F>* __restrict__ bu
 constexpr int WTREE = 64;
 template <class F>
 __global__ void __launch_bounds__(256) k_wtree(const XYZZ<F>* __restrict__ u_in, const XYZZ<F>* __restrict__ v_in,
-                                               uint32_t S, XYZZ<F>* __restrict__ u_out, XYZZ<F>* __restrict__ v_out) {
+                                               uint32_t S, XYZZ<F>* __restrict__ u_out, XYZZ<F>* __restrict__ v_out,
+                                               const uint32_t* bad, const uint32_t* points_bad, uint32_t* host_bad) {
     __shared__ F sh[2 * WTREE][4];  // U, then V
     const uint32_t nblk = S > (uint32_t)WTREE ? S / WTREE : 1u;
     const uint32_t w = blockIdx.x / nblk, k = blockIdx.x % nblk;
@@ -849,6 +850,10 @@ __global__ void __launch_bounds__(256) k_wtree(const XYZZ<F>* __restrict__ u_in,
     if (threadIdx.x < 4) {
         reinterpret_cast<F*>(u_out)[(size_t)blockIdx.x * 4 + r] = sh[0][r];
         if (nblk > 1) reinterpret_cast<F*>(v_out)[(size_t)blockIdx.x * 4 + r] = sh[WTREE][r];
+    }
+    if (host_bad && blockIdx.x == 0 && threadIdx.x == 0) {
+        host_bad[0] = *bad;
+        host_bad[1] = points_bad ? *points_bad : NO_INDEX;
     }
 }
 
@@ -1203,7 +1208,8 @@ void accumulate(MsmWorkspace& ws, const Affine<F>* pts, const uint32_t* d_sorted
 
 template <class F>
 void msm_enqueue(MsmWorkspace& ws, const Affine<F>* d_points, const uint32_t* d_scalars, const SetMap& map,
-                 uint32_t n, const MsmPlan& plan, const MsmPrecomp<F>* pre, uint32_t* d_err, cudaStream_t st) {
+                 uint32_t n, const MsmPlan& plan, const MsmPrecomp<F>* pre, uint32_t* d_err, cudaStream_t st,
+                 const MsmHost<F>* host) {
     const uint32_t count = map.count;
     const int c = plan.c, W = plan.windows;
     const uint32_t B = plan.buckets;
@@ -1259,7 +1265,7 @@ void msm_enqueue(MsmWorkspace& ws, const Affine<F>* d_points, const uint32_t* d_
     XYZZ<F>* d_seg_r = d_seg_u + (size_t)NW * S;
     XYZZ<F>* d_lvl_u = d_seg_r + (size_t)NW * S;  // ping-pong buffers of the upper levels
     XYZZ<F>* d_lvl_r = d_lvl_u + (size_t)NW * S;
-    XYZZ<F>* d_win = ws.windows.as<XYZZ<F>>(NW);
+    XYZZ<F>* d_win = host ? host->windows : ws.windows.as<XYZZ<F>>(NW);
 
     if (tl.enabled) DV_CUDA(cudaEventRecord(tl.acc_ev[0], st));
     accumulate<F>(ws, pre ? pre->table : d_points, d_sorted, d_offsets, NB, (uint64_t)n * W, d_buckets, st);
@@ -1276,7 +1282,8 @@ void msm_enqueue(MsmWorkspace& ws, const Affine<F>* d_points, const uint32_t* d_
     for (;;) {
         const uint32_t nblk = len > (uint32_t)WTREE ? len / WTREE : 1u;
         XYZZ<F>* u_dst = nblk == 1 ? d_win : u2;
-        k_wtree<F><<<NW * nblk, 256, 0, st>>>(u, r, len, u_dst, r2);
+        k_wtree<F><<<NW * nblk, 256, 0, st>>>(u, r, len, u_dst, r2, d_err, host ? host->d_points_bad : nullptr,
+                                              host && nblk == 1 ? host->bad : nullptr);
         DV_LAUNCH();
         if (nblk == 1) break;
         len = nblk;
@@ -1289,7 +1296,7 @@ void msm_enqueue(MsmWorkspace& ws, const Affine<F>* d_points, const uint32_t* d_
 template <class F>
 void msm_run(MsmWorkspace& ws, const Affine<F>* d_points, const uint32_t* d_scalars, const uint32_t* set_offsets,
              uint32_t count, int force_c, cudaStream_t st, uint8_t* host_out, MsmStats* stats,
-             const MsmPrecomp<F>* pre) {
+             const MsmPrecomp<F>* pre, const uint32_t* d_points_bad, uint32_t* points_bad) {
     typedef typename HostOf<F>::T HF;
     const size_t out_bytes = 2 * sizeof(F);
     const uint32_t n = set_offsets[count];
@@ -1306,18 +1313,16 @@ void msm_run(MsmWorkspace& ws, const Affine<F>* d_points, const uint32_t* d_scal
 
     uint32_t* d_set = ws.set_off.as<uint32_t>(count + 1);
     uint32_t* d_err = ws.err.as<uint32_t>(1);
-    uint32_t* h_err = ws.host_err.as<uint32_t>(1);
+    uint32_t* h_err = ws.host_err.as<uint32_t>(2);
     DV_CUDA(cudaMemcpyAsync(d_set, set_offsets, (count + 1) * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
     DV_CUDA(cudaMemsetAsync(d_err, 0xff, sizeof(uint32_t), st));
-    msm_enqueue<F>(ws, d_points, d_scalars, SetMap{d_set, nullptr, count, 0}, n, plan, pre, d_err, st);
-
     XYZZ<F>* h_win = ws.host_windows.as<XYZZ<F>>(NW);
-    DV_CUDA(cudaMemcpyAsync(h_win, ws.windows.as<XYZZ<F>>(NW), (size_t)NW * sizeof(XYZZ<F>), cudaMemcpyDeviceToHost,
-                            st));
-    DV_CUDA(cudaMemcpyAsync(h_err, d_err, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+    const MsmHost<F> host{h_win, d_points_bad, h_err};
+    msm_enqueue<F>(ws, d_points, d_scalars, SetMap{d_set, nullptr, count, 0}, n, plan, pre, d_err, st, &host);
     DV_CUDA(cudaStreamSynchronize(st));
     if (*h_err != NO_INDEX)
         throw InvalidArgument("non-canonical scalar at index " + std::to_string(*h_err));
+    if (points_bad) *points_bad = h_err[1];
     static_assert(sizeof(XYZZ<F>) == sizeof(dvh::XYZZ<HF>), "host/device XYZZ layout");
     const auto* hw = reinterpret_cast<const dvh::XYZZ<HF>*>(h_win);
     for (uint32_t k = 0; k < count; ++k) horner(hw + (size_t)k * Wr, (int)Wr, c, host_out + (size_t)k * out_bytes);
@@ -1505,15 +1510,15 @@ void msm_sparse_direct(MsmWorkspace& ws, const MsmPrecomp<Fq>& pre, uint64_t nba
 }
 
 template void msm_run<Fq>(MsmWorkspace&, const Affine<Fq>*, const uint32_t*, const uint32_t*, uint32_t, int,
-                          cudaStream_t, uint8_t*, MsmStats*, const MsmPrecomp<Fq>*);
+                          cudaStream_t, uint8_t*, MsmStats*, const MsmPrecomp<Fq>*, const uint32_t*, uint32_t*);
 template void msm_run<Fq2>(MsmWorkspace&, const Affine<Fq2>*, const uint32_t*, const uint32_t*, uint32_t, int,
-                           cudaStream_t, uint8_t*, MsmStats*, const MsmPrecomp<Fq2>*);
+                           cudaStream_t, uint8_t*, MsmStats*, const MsmPrecomp<Fq2>*, const uint32_t*, uint32_t*);
 template MsmPlan msm_plan_batch<Fq>(uint32_t, uint32_t, uint64_t, int, const MsmPrecomp<Fq>*);
 template MsmPlan msm_plan_batch<Fq2>(uint32_t, uint32_t, uint64_t, int, const MsmPrecomp<Fq2>*);
 template void msm_enqueue<Fq>(MsmWorkspace&, const Affine<Fq>*, const uint32_t*, const SetMap&, uint32_t,
-                              const MsmPlan&, const MsmPrecomp<Fq>*, uint32_t*, cudaStream_t);
+                              const MsmPlan&, const MsmPrecomp<Fq>*, uint32_t*, cudaStream_t, const MsmHost<Fq>*);
 template void msm_enqueue<Fq2>(MsmWorkspace&, const Affine<Fq2>*, const uint32_t*, const SetMap&, uint32_t,
-                               const MsmPlan&, const MsmPrecomp<Fq2>*, uint32_t*, cudaStream_t);
+                               const MsmPlan&, const MsmPrecomp<Fq2>*, uint32_t*, cudaStream_t, const MsmHost<Fq2>*);
 
 template <class F>
 void msm_finish_device(const XYZZ<F>* d_windows, uint32_t count, int windows_per_set, int c, const uint32_t* d_out_idx,

@@ -106,10 +106,24 @@ void msm_sparse_direct(MsmWorkspace& ws, const MsmPrecomp<Fq>& pre, uint64_t nba
 // pipeline 235 us for 256 entries, 202 and 219 for 512, 335 and 227 for 1024.
 constexpr uint64_t SPARSE_DIRECT_MAX_TERMS = 1u << 14;
 
+// *d_points_bad, the error word of the points' conversion in the same stream,
+// is read before the wait and left in *points_bad.
 template <class F>
 void msm_run(MsmWorkspace& ws, const Affine<F>* d_points, const uint32_t* d_scalars, const uint32_t* set_offsets,
              uint32_t count, int force_c, cudaStream_t stream, uint8_t* host_out, MsmStats* stats,
-             const MsmPrecomp<F>* pre = nullptr);
+             const MsmPrecomp<F>* pre = nullptr, const uint32_t* d_points_bad = nullptr,
+             uint32_t* points_bad = nullptr);
+
+// Where the last reduction kernel of a launch sequence that the host waits for
+// leaves its results: pinned host memory, written by the kernel.  A copy
+// behind it and the wait for that copy take 6 us each, which a call of a
+// thousand points notices (from host memory 273 -> 253 us without).
+template <class F>
+struct MsmHost {
+    XYZZ<F>* windows;              // as ws.windows
+    const uint32_t* d_points_bad;  // error word of the conversion, device, or null
+    uint32_t* bad;                 // the scalars' error word, then the conversion's
+};
 
 // How the digits of one launch sequence map to sets, scalars and points.
 // Digit i (0 <= i < off[count]) belongs to the set k with
@@ -139,13 +153,15 @@ MsmPlan msm_plan_batch(uint32_t count, uint32_t max_set, uint64_t total, int for
 // The device part of an MSM launch sequence: digit sort, accumulation,
 // merges and bucket reduction, all on `stream`, without host
 // synchronisation.  Leaves count * (pre ? 1 : windows) XYZZ window sums in
-// ws.windows and the lowest non-canonical scalar index (or 0xffffffff) in
-// *d_err, which the caller initialises.  Allocates only when a workspace
+// ws.windows (with host: there instead, and the error words) and the lowest
+// non-canonical scalar index (or 0xffffffff) in *d_err, which the caller
+// initialises.  Allocates only when a workspace
 // buffer must grow, so a second call with the same shapes allocates nothing
 // (and can be captured in a CUDA graph).
 template <class F>
 void msm_enqueue(MsmWorkspace& ws, const Affine<F>* d_points, const uint32_t* d_scalars, const SetMap& map,
-                 uint32_t n, const MsmPlan& plan, const MsmPrecomp<F>* pre, uint32_t* d_err, cudaStream_t stream);
+                 uint32_t n, const MsmPlan& plan, const MsmPrecomp<F>* pre, uint32_t* d_err, cudaStream_t stream,
+                 const MsmHost<F>* host = nullptr);
 
 // Device tail: Horner over each set's window sums (weights 2^(c w)) and
 // normalisation to canonical affine bytes (2 * sizeof(F) per set, all-zero
