@@ -421,3 +421,30 @@ def test_msm_error_words_reach_the_host(dv, backend, oracle, n, g2):
                 call(p, s)
             assert e.value.status == -1 and message in e.value.message
             assert call(pts, scs) == expect
+
+
+def test_sparse_direct_error_words_of_several_requests(dv, backend, oracle):
+    """Each request's last block hands its error words to the host: the lowest
+    bad scalar of all requests is named, empty requests give infinity, and the
+    next call is good."""
+    n, offs = 64, [0, 0, 3, 3, 12, 30, 30]
+    bases = oracle.fixed_base_g1(oracle.uniform_fr(8200, n))
+    idx = (np.arange(offs[-1], dtype=np.uint64) * 7) % n
+    vals = oracle.uniform_fr(8201, offs[-1])
+    r = (0x30644E72E131A029B85045B68181585D2833E84879B9709143E1F593F0000001).to_bytes(32, "little")
+    expect = [oracle.sparse_msm_g1(bases, idx[a:b], vals[32 * a:32 * b]) if b > a else bytes(64)
+              for a, b in zip(offs, offs[1:])]
+    h = backend.register_bases(bases)
+    try:
+        backend.precompute_bases(h, 8)
+        assert backend.sparse_msm_resident(h, idx, vals, offs) == expect
+        for bad in ([29], [2, 29], [11, 12], [0]):
+            broken = bytearray(vals)
+            for at in bad:
+                broken[32 * at:32 * at + 32] = r
+            with pytest.raises(dv.DvgpuError) as e:
+                backend.sparse_msm_resident(h, idx, bytes(broken), offs)
+            assert e.value.status == -1 and f"non-canonical scalar at index {min(bad)}" in e.value.message
+            assert backend.sparse_msm_resident(h, idx, vals, offs) == expect
+    finally:
+        backend.release_bases(h)

@@ -1385,12 +1385,13 @@ DV_INL Fq quads_sum_block(Fq acc, Fq (*sh)[4]) {
 // SD_TERMS (entry, window) terms of one request: a lane quad forms d T (the
 // signed c-bit digit d of the entry's window, T the table's multiple
 // 2^(c w) P) by double-and-add, the block sums its quads.  The last block
-// of a request to finish (a per-request counter, reset by that block for the
-// next call) sums the request's block partials and writes the XYZZ sum.
+// of a request to finish (a per-request counter) sums the request's block partials and writes the XYZZ sum
+// and the error words to pinned memory.
 // The launch is one chain: up to c doublings and c / 2 additions, a tree of
 // six additions, the same over the partials, each three or four dependent
 // products in a quad.  256 entries of 32 windows, a whole call from host
-// memory: 210 us with a thread a term and one bit a step, 143 us so.
+// memory: 210 us with a thread a term and one bit a step, 137 us so, 125
+// without fills and copies beside the kernel.
 // The host normalises all requests with one batch inversion, as the
 // reference does (icicle_msm.cu:417-421): one thread's inversion on the
 // device takes longer than that copy and a host batch inversion.
@@ -1400,7 +1401,8 @@ __global__ void __launch_bounds__(SD_THREADS) k_sparse_direct(const G1A* __restr
                                                             const SdJob* __restrict__ jobs,
                                                             const uint32_t* __restrict__ req_blocks,
                                                             XYZZ<Fq>* __restrict__ partial, uint32_t* __restrict__ done,
-                                                            XYZZ<Fq>* __restrict__ out, uint32_t* __restrict__ err) {
+                                                            XYZZ<Fq>* __restrict__ out, uint32_t* __restrict__ err,
+                                                             uint32_t* __restrict__ host_err) {
     __shared__ Fq sh[SD_THREADS / 32][4];
     __shared__ bool last;
     const SdJob job = jobs[blockIdx.x];
@@ -1448,7 +1450,10 @@ __global__ void __launch_bounds__(SD_THREADS) k_sparse_direct(const G1A* __restr
         __threadfence();
     }
     __syncthreads();
-    if (threadIdx.x == 0) last = atomicAdd(done + req, 1u) == b1 - b0 - 1;
+    if (threadIdx.x == 0) {
+        __threadfence();  // the block's error words
+        last = atomicAdd(done + req, 1u) == b1 - b0 - 1;
+    }
     __syncthreads();
     if (!last) return;
     __threadfence();
@@ -1457,7 +1462,8 @@ __global__ void __launch_bounds__(SD_THREADS) k_sparse_direct(const G1A* __restr
         p = Quad<Fq>::add(p, b < b1 ? load_cg(reinterpret_cast<const Fq*>(partial + b) + r) : Quad<Fq>::inf());
     p = quads_sum_block(p, sh);
     if (threadIdx.x < 4) reinterpret_cast<Fq*>(out + req)[r] = p;
-    if (threadIdx.x == 0) done[req] = 0;
+    // at least the errors of this request; the host takes the least of all
+    if (threadIdx.x < 2) host_err[2 * req + threadIdx.x] = static_cast<volatile const uint32_t*>(err)[threadIdx.x];
 }
 
 void msm_sparse_direct(MsmWorkspace& ws, const MsmPrecomp<Fq>& pre, uint64_t nbases, const uint64_t* d_idx,
@@ -1478,31 +1484,33 @@ void msm_sparse_direct(MsmWorkspace& ws, const MsmPrecomp<Fq>& pre, uint64_t nba
         memset(host_out, 0, (size_t)count * 64);
         return;
     }
-    // one upload: the block list, then the per-request block offsets
-    const size_t jb = jobs.size() * sizeof(SdJob), rb = (count + 1) * sizeof(uint32_t);
-    uint8_t* h_desc = ws.host_desc.as<uint8_t>(jb + rb);
+    // one upload: the block list, the per-request block offsets, the
+    // requests' counters and the error words; the kernel writes sums and
+    // error words to pinned memory, so nothing is copied or set beside it
+    // (two fills and a copy back before)
+    const size_t jb = jobs.size() * sizeof(SdJob), rb = (count + 1) * sizeof(uint32_t), cb = count * sizeof(uint32_t);
+    uint8_t* h_desc = ws.host_desc.as<uint8_t>(jb + rb + cb + 8);
     memcpy(h_desc, jobs.data(), jb);
     memcpy(h_desc + jb, req_blocks.data(), rb);
-    uint8_t* d_desc = ws.sd_jobs.as<uint8_t>(jb + rb);
+    memset(h_desc + jb + rb, 0, cb);
+    memset(h_desc + jb + rb + cb, 0xff, 8);
+    uint8_t* d_desc = ws.sd_jobs.as<uint8_t>(jb + rb + cb + 8);
+    uint32_t* d_done = reinterpret_cast<uint32_t*>(d_desc + jb + rb);
     XYZZ<Fq>* d_partial = ws.sd_partial.as<XYZZ<Fq>>(jobs.size());
-    uint32_t* d_done = ws.sd_req.as<uint32_t>(count);
     constexpr size_t XB = sizeof(XYZZ<Fq>);
-    uint8_t* d_out = ws.sd_out.as<uint8_t>((size_t)count * XB + 16);
-    uint32_t* d_err = reinterpret_cast<uint32_t*>(d_out + (size_t)count * XB);
-    DV_CUDA(cudaMemcpyAsync(d_desc, h_desc, jb + rb, cudaMemcpyHostToDevice, st));
-    DV_CUDA(cudaMemsetAsync(d_done, 0, count * sizeof(uint32_t), st));
-    if (empty) DV_CUDA(cudaMemsetAsync(d_out, 0, (size_t)count * XB, st));  // all-zero XYZZ: infinity
-    DV_CUDA(cudaMemsetAsync(d_err, 0xff, 2 * sizeof(uint32_t), st));
+    uint8_t* h_out = ws.host_windows.as<uint8_t>((size_t)count * (XB + 8));
+    if (empty) memset(h_out, 0, (size_t)count * XB);  // all-zero XYZZ: infinity
+    uint32_t* h_words = reinterpret_cast<uint32_t*>(h_out + (size_t)count * XB);
+    memset(h_words, 0xff, (size_t)count * 8);
+    DV_CUDA(cudaMemcpyAsync(d_desc, h_desc, jb + rb + cb + 8, cudaMemcpyHostToDevice, st));
     k_sparse_direct<<<(unsigned)jobs.size(), SD_THREADS, 0, st>>>(
         pre.table, nbases, pre.c, (int)W, d_idx, d_vals, reinterpret_cast<const SdJob*>(d_desc),
-        reinterpret_cast<const uint32_t*>(d_desc + jb), d_partial, d_done, reinterpret_cast<XYZZ<Fq>*>(d_out), d_err);
+        reinterpret_cast<const uint32_t*>(d_desc + jb), d_partial, d_done, reinterpret_cast<XYZZ<Fq>*>(h_out),
+        d_done + count, h_words);
     DV_LAUNCH();
-    // one copy back: the results, then the two error words
-    uint8_t* h_out = ws.host_windows.as<uint8_t>((size_t)count * XB + 16);
-    DV_CUDA(cudaMemcpyAsync(h_out, d_out, (size_t)count * XB + 8, cudaMemcpyDeviceToHost, st));
     DV_CUDA(cudaStreamSynchronize(st));
-    uint32_t h_err[2];
-    memcpy(h_err, h_out + (size_t)count * XB, 8);
+    uint32_t h_err[2] = {NO_INDEX, NO_INDEX};
+    for (uint32_t k = 0; k < 2 * count; ++k) h_err[k & 1] = std::min(h_err[k & 1], h_words[k]);
     if (h_err[0] != NO_INDEX) throw InvalidArgument("non-canonical scalar at index " + std::to_string(h_err[0]));
     if (h_err[1] != NO_INDEX) throw InvalidArgument("sparse MSM index out of range");
     static_assert(sizeof(XYZZ<Fq>) == sizeof(dvh::XYZZ<dvh::Fq>), "host/device XYZZ layout");
