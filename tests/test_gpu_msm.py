@@ -380,6 +380,35 @@ def test_msm_repeated_scalars(backend, oracle, n, g2):
         assert run(pts, s.to_bytes(32, "little") * n) == expect, s
 
 
+def _collected_sum(oracle, bases, sc):
+    """sum sc_i bases_(i mod len(bases)) from the sums of each base's scalars."""
+    m = len(bases)
+    r = 0x30644E72E131A029B85045B68181585D2833E84879B9709143E1F593F0000001
+    limbs = np.frombuffer(sc, dtype="<u4").reshape(-1, 8).astype(np.uint64)
+    sums = [sum(int(x) << (32 * k) for k, x in enumerate(limbs[i::m].sum(axis=0))) % r for i in range(m)]
+    return oracle.msm_g1(b"".join(bases), b"".join(x.to_bytes(32, "little") for x in sums))
+
+
+@pytest.mark.parametrize("c", [8, 13, 16])
+def test_msm_many_long_chains(backend, oracle, c):
+    """Queues of long bucket chains over a window table: some hundred of block
+    length (c = 8), thousands of warp length, more than one round of the queue
+    (c = 13), and with one value everywhere one a window, among short ones
+    with half the scalars equal."""
+    n = 40000
+    srs, _ = oracle.srs_g1(6301, 64)
+    bases = [srs[64 * i:64 * i + 64] for i in range(64)]
+    h = backend.register_bases((srs * (n // 64 + 1))[:64 * n])
+    try:
+        backend.precompute_bases(h, c)
+        uniform, one = oracle.uniform_fr(6302, n), oracle.uniform_fr(6303, 1)
+        half = b"".join(one if i % 2 else uniform[32 * i:32 * i + 32] for i in range(n))
+        for sc in (uniform, one * n, half):
+            assert backend.msm_resident_host(h, sc) == _collected_sum(oracle, bases, sc)
+    finally:
+        backend.release_bases(h)
+
+
 @pytest.mark.parametrize("c", [8, 13])
 def test_sparse_direct_block_edges(backend, oracle, c):
     """One request around a block's 64 terms and around the direct path's
