@@ -409,6 +409,22 @@ def test_msm_many_long_chains(backend, oracle, c):
         backend.release_bases(h)
 
 
+@pytest.mark.parametrize("value", [0, 1, 255])
+def test_msm_of_nearly_empty_lists(backend, oracle, value):
+    """Plans with pairwise levels and next to nothing to sum: no digit at all,
+    one entry, and the levels' least list of 4096 entries (value 1) from both
+    sides; empty trees, and trees of one full bucket among empty ones."""
+    n = 230001
+    srs, _ = oracle.srs_g1(6401, 64)
+    bases = [srs[64 * i:64 * i + 64] for i in range(64)]
+    pts = (srs * (n // 64 + 1))[:64 * n]
+    for k in (0, 1, 4095, 4096, 4097):
+        sc = bytearray(32 * n)
+        for i in range(k):
+            sc[32 * (53 * i % n)] = value
+        assert backend.msm(pts, bytes(sc)) == _collected_sum(oracle, bases, bytes(sc)), k
+
+
 @pytest.mark.parametrize("c", [8, 13])
 def test_sparse_direct_block_edges(backend, oracle, c):
     """One request around a block's 64 terms and around the direct path's

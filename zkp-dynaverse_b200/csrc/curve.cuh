@@ -232,7 +232,9 @@ DV_INL F warp_batch_inverse(const F& x) {
 // zz, zzz): an addition is four dependent products instead of a lane's
 // fourteen, a doubling three instead of nine, for chains of few points (a
 // quarter more multiply-adds a point when lanes are not free).  Every lane of
-// the warp takes part; quads without work hold infinity.
+// the warp takes part; quads without work hold infinity.  A warp none of whose
+// quads has two points to add skips the products: empty buckets (short or small
+// scalars) then cost no more than with a thread a point.
 template <class F>
 struct Quad {
     F c;
@@ -261,6 +263,7 @@ struct Quad {
     static __device__ __noinline__ F add(F p, F q) {
         const int r = role();
         const bool pi = flag(p.is_zero(), 2), qi = flag(q.is_zero(), 2);
+        if (__all_sync(0xffffffffu, pi || qi)) return pi ? q : p;
         const F t = F::mul(p, shfl_xor(q, 2));             // U1, S1, U2, S2
         const F o = shfl_xor(t, 2);
         const F d = r < 2 ? F::sub(o, t) : F::sub(t, o);   // P on lanes 0, 2; R on 1, 3

@@ -362,7 +362,10 @@ struct PairCaps {
 DV_INL uint32_t pair_start(const uint32_t* offsets, uint32_t g) { return (uint32_t)(((uint64_t)offsets[g] + g) >> 1); }
 
 // Chunks of about equal slots, cut at buckets; pairs = 0 where one does not
-// fit its room (digits far from uniform).
+// fit its room (digits far from uniform) or holds next to nothing (scalars that
+// are nearly all zero; 4096 entries are one addition a thread in k_accum, and
+// in one bucket still only 64 merges in a row, less than the levels take).
+constexpr uint32_t PAIR_LEAST = 4096;
 __global__ void k_pair_chunks(const uint32_t* __restrict__ offsets, uint32_t nb, uint32_t chunks, int levels,
                               const PairCaps caps, AccumChunk* __restrict__ out) {
     const uint32_t c = threadIdx.x;
@@ -380,7 +383,7 @@ __global__ void k_pair_chunks(const uint32_t* __restrict__ offsets, uint32_t nb,
     }
     const uint32_t n = bound[1] - bound[0];
     uint64_t slots = offsets[bound[1]] - offsets[bound[0]];
-    bool fits = n > 0;
+    bool fits = n > 0 && slots >= PAIR_LEAST;
     uint32_t first = 0;
     for (int k = 0; k < levels; ++k) {
         slots = (slots + n) >> 1;
@@ -845,7 +848,7 @@ __global__ void __launch_bounds__(256) k_wtree(const XYZZ<F>* __restrict__ u_in,
             const bool live = is_u || is_v;
             s = Quad<F>::add(live ? x[(2 * j) * 4 + r] : Quad<F>::inf(), live ? x[(2 * j + 1) * 4 + r] : Quad<F>::inf());
             if (warp_u) s = Quad<F>::add(s, is_u ? sh[WTREE + 2 * j + 1][r] : Quad<F>::inf());
-            else s = Quad<F>::dbl(s);
+            else if (__any_sync(0xffffffffu, r == 2 && !s.is_zero())) s = Quad<F>::dbl(s);
         }
         __syncthreads();
         if (is_u) sh[j][r] = s;
