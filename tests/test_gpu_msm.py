@@ -444,6 +444,45 @@ def test_sparse_direct_block_edges(backend, oracle, c):
         backend.release_bases(h)
 
 
+@pytest.mark.parametrize("c, requests, entries, direct",
+                         [(8, 300, 4, True), (8, 70, 16, True), (8, 1100, 1, True), (8, 2, 900, False),
+                          (8, 40, 75, False), (13, 300, 4, True), (13, 70, 16, True), (13, 1100, 1, True),
+                          (13, 40, 75, True), (13, 2, 900, False)])
+def test_sparse_many_requests(dv, backend, oracle, c, requests, entries, direct):
+    """Calls of many requests between 16384 and 65536 terms stay one launch
+    (blocks of quads for the shortest requests, of threads for the others), with
+    empty requests, repeated indices and error words; few requests and
+    more terms take the buckets."""
+    n, r = 256, 0x30644E72E131A029B85045B68181585D2833E84879B9709143E1F593F0000001
+    bases = oracle.fixed_base_g1(oracle.uniform_fr(8300, n))
+    sizes = [0 if j % 17 == 5 else entries + j % 2 for j in range(requests)]
+    offs = [0] + list(np.cumsum(sizes))
+    k = int(offs[-1])
+    idx = (np.arange(k, dtype=np.uint64) * 5 + 3) % n
+    vals = bytearray(oracle.uniform_fr(8301, k))
+    vals[64:96] = bytes(32)
+    vals[96:128] = (r - 1).to_bytes(32, "little")
+    vals = bytes(vals)
+    expect = [oracle.sparse_msm_g1(bases, idx[a:b], vals[32 * a:32 * b]) if b > a else bytes(64)
+              for a, b in zip(offs, offs[1:])]
+    h = backend.register_bases(bases)
+    try:
+        backend.precompute_bases(h, c)
+        before = backend.launch_count()
+        assert backend.sparse_msm_resident(h, idx, vals, offs) == expect
+        assert (backend.launch_count() - before == 1) == direct
+        for bad in ([k - 1], [k // 2, k - 1], [0]):
+            broken = bytearray(vals)
+            for at in bad:
+                broken[32 * at:32 * at + 32] = r.to_bytes(32, "little")
+            with pytest.raises(dv.DvgpuError) as e:
+                backend.sparse_msm_resident(h, idx, bytes(broken), offs)
+            assert e.value.status == -1 and f"non-canonical scalar at index {min(bad)}" in e.value.message
+        assert backend.sparse_msm_resident(h, idx, vals, offs) == expect
+    finally:
+        backend.release_bases(h)
+
+
 @pytest.mark.parametrize("n", [1, 300, 5000])
 @pytest.mark.parametrize("g2", [False, True])
 def test_msm_error_words_reach_the_host(dv, backend, oracle, n, g2):

@@ -1389,6 +1389,45 @@ DV_INL Fq quads_sum_block(Fq acc, Fq (*sh)[4]) {
     return acc;
 }
 
+// Tree sum of sm[0 .. live) into sm[0] (entries up to the next power of two
+// hold infinity): only the levels the live entries need.
+DV_INL void block_sum(XYZZ<Fq>* sm, uint32_t live) {
+    uint32_t span = 1;
+    while (span < live) span <<= 1;
+    for (uint32_t stride = span >> 1; stride > 0; stride >>= 1) {
+        if (threadIdx.x < stride) sm[threadIdx.x] = XYZZ<Fq>::add_paired(sm[threadIdx.x], sm[threadIdx.x + stride]);
+        __syncthreads();
+    }
+}
+
+// Term `term` of a sparse MSM: its table entry with the digit's sign in
+// `point`; returns the digit's magnitude, 0 where nothing is to be added (a
+// non-canonical scalar and an index out of range are noted in err).
+DV_INL uint32_t sparse_term(const G1A* __restrict__ table, uint64_t nbases, int c, int W,
+                            const uint64_t* __restrict__ idx, const uint32_t* __restrict__ vals, uint32_t term,
+                            uint32_t* __restrict__ err, G1A& point) {
+    const uint32_t e = term / (uint32_t)W, w = term % (uint32_t)W;
+    uint32_t s[8];
+    load_scalar(vals, e, s);
+    const uint64_t ix = idx[e];
+    if (!Fr::is_canonical(s)) {
+        if (w == 0) atomicMin(err, e);
+        return 0;
+    }
+    if (ix >= nbases) {
+        if (w == 0) atomicMin(err + 1, e);
+        return 0;
+    }
+    // signed digit of window w (the recoding of k_hist)
+    const uint32_t B = 1u << (c - 1), full = 1u << c;
+    const uint32_t* words = vals + 8ull * e;
+    const uint32_t d = window_raw(words, (int)w * c, c) + carry_into(words, (int)w, c);
+    const bool neg = d > B;
+    point = table[ix * (uint64_t)W + w];
+    if (neg) point.y = Fq::neg(point.y);
+    return point.is_inf() ? 0u : neg ? full - d : d;
+}
+
 // Sparse MSMs over a window table in one launch.  Each block takes up to
 // SD_TERMS (entry, window) terms of one request: a lane quad forms d T (the
 // signed c-bit digit d of the entry's window, T the table's multiple
@@ -1403,13 +1442,13 @@ DV_INL Fq quads_sum_block(Fq acc, Fq (*sh)[4]) {
 // The host normalises all requests with one batch inversion, as the
 // reference does (icicle_msm.cu:417-421): one thread's inversion on the
 // device takes longer than that copy and a host batch inversion.
-__global__ void __launch_bounds__(SD_THREADS) k_sparse_direct(const G1A* __restrict__ table, uint64_t nbases, int c,
-                                                            int W, const uint64_t* __restrict__ idx,
-                                                            const uint32_t* __restrict__ vals,
-                                                            const SdJob* __restrict__ jobs,
-                                                            const uint32_t* __restrict__ req_blocks,
-                                                            XYZZ<Fq>* __restrict__ partial, uint32_t* __restrict__ done,
-                                                            XYZZ<Fq>* __restrict__ out, uint32_t* __restrict__ err,
+__global__ void __launch_bounds__(SD_THREADS) k_sparse_quads(const G1A* __restrict__ table, uint64_t nbases, int c,
+                                                             int W, const uint64_t* __restrict__ idx,
+                                                             const uint32_t* __restrict__ vals,
+                                                             const SdJob* __restrict__ jobs,
+                                                             const uint32_t* __restrict__ req_blocks,
+                                                             XYZZ<Fq>* __restrict__ partial, uint32_t* __restrict__ done,
+                                                             XYZZ<Fq>* __restrict__ out, uint32_t* __restrict__ err,
                                                              uint32_t* __restrict__ host_err) {
     __shared__ Fq sh[SD_THREADS / 32][4];
     __shared__ bool last;
@@ -1418,25 +1457,9 @@ __global__ void __launch_bounds__(SD_THREADS) k_sparse_direct(const G1A* __restr
     uint32_t mag = 0;
     Fq t = Quad<Fq>::inf();
     if (quad < job.items) {
-        const uint32_t term = job.first + quad;
-        const uint32_t e = term / (uint32_t)W, w = term % (uint32_t)W;
-        uint32_t s[8];
-        load_scalar(vals, e, s);
-        const uint64_t ix = idx[e];
-        if (!Fr::is_canonical(s)) {
-            if (w == 0) atomicMin(err, e);
-        } else if (ix >= nbases) {
-            if (w == 0) atomicMin(err + 1, e);
-        } else {
-            // signed digit of window w (the recoding of k_hist)
-            const uint32_t B = 1u << (c - 1), full = 1u << c;
-            const uint32_t* words = vals + 8ull * e;
-            const uint32_t d = window_raw(words, (int)w * c, c) + carry_into(words, (int)w, c);
-            const bool neg = d > B;
-            const G1A a = table[ix * (uint64_t)W + w];
-            mag = a.is_inf() ? 0u : neg ? full - d : d;
-            if (mag) t = r == 0 ? a.x : r == 1 ? (neg ? Fq::neg(a.y) : a.y) : Fq::one();
-        }
+        G1A a;
+        mag = sparse_term(table, nbases, c, W, idx, vals, job.first + quad, err, a);
+        if (mag) t = r == 0 ? a.x : r == 1 ? a.y : Fq::one();
     }
     // d T by two bits a step over T, 2 T, 3 T, from each quad's top pair of
     // bits on, the warp in step with its longest digit
@@ -1474,17 +1497,81 @@ __global__ void __launch_bounds__(SD_THREADS) k_sparse_direct(const G1A* __restr
     if (threadIdx.x < 2) host_err[2 * req + threadIdx.x] = static_cast<volatile const uint32_t*>(err)[threadIdx.x];
 }
 
+// The same with a thread per term and blocks of four times the terms, for
+// calls of many requests whose quads would take several waves: a quad is the
+// shorter chain, but a quarter more multiply-adds.
+__global__ void __launch_bounds__(SD_THREADS) k_sparse_threads(const G1A* __restrict__ table, uint64_t nbases, int c,
+                                                               int W, const uint64_t* __restrict__ idx,
+                                                               const uint32_t* __restrict__ vals,
+                                                               const SdJob* __restrict__ jobs,
+                                                               const uint32_t* __restrict__ req_blocks,
+                                                               XYZZ<Fq>* __restrict__ partial,
+                                                               uint32_t* __restrict__ done, XYZZ<Fq>* __restrict__ out,
+                                                               uint32_t* __restrict__ err,
+                                                               uint32_t* __restrict__ host_err) {
+    __shared__ XYZZ<Fq> sm[SD_THREADS];
+    __shared__ bool last;
+    const SdJob job = jobs[blockIdx.x];
+    const uint32_t t = threadIdx.x;
+    XYZZ<Fq> p = XYZZ<Fq>::inf();
+    if (t < job.items) {
+        G1A a;
+        const uint32_t mag = sparse_term(table, nbases, c, W, idx, vals, job.first + t, err, a);
+        if (mag) {
+            p = XYZZ<Fq>::from_affine(a);
+            for (int b = 30 - __clz(mag); b >= 0; --b) {
+                p = XYZZ<Fq>::dbl_paired(p);
+                if ((mag >> b) & 1) p = XYZZ<Fq>::add_affine(p, a);
+            }
+        }
+    }
+    sm[t] = p;
+    __syncthreads();
+    block_sum(sm, job.items);
+    const uint32_t req = job.request, b0 = req_blocks[req], b1 = req_blocks[req + 1];
+    if (t == 0) {
+        partial[blockIdx.x] = sm[0];
+        __threadfence();  // and the block's error words
+        last = atomicAdd(done + req, 1u) == b1 - b0 - 1;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    p = XYZZ<Fq>::inf();
+    for (uint32_t b = b0 + t; b < b1; b += SD_THREADS) {
+        const Fq* q = reinterpret_cast<const Fq*>(partial + b);
+        p = XYZZ<Fq>::add_paired(p, {load_cg(q), load_cg(q + 1), load_cg(q + 2), load_cg(q + 3)});
+    }
+    sm[t] = p;
+    __syncthreads();
+    block_sum(sm, min(b1 - b0, (uint32_t)SD_THREADS));
+    if (t == 0) out[req] = sm[0];
+    if (t < 2) host_err[2 * req + t] = static_cast<volatile const uint32_t*>(err)[t];
+}
+
 void msm_sparse_direct(MsmWorkspace& ws, const MsmPrecomp<Fq>& pre, uint64_t nbases, const uint64_t* d_idx,
                        const uint32_t* d_vals, const uint32_t* offs, uint32_t count, uint8_t* host_out,
                        cudaStream_t st) {
     const uint32_t W = (uint32_t)pre.windows;
+    // Quads while they are one wave of blocks, or where requests are so short
+    // that threads would leave blocks mostly empty (32768 terms over a c = 8
+    // table: one request 327 us by quads and 227 by threads, 256 requests 383 and
+    // 348, 1024 requests 726 and 1027).
+    uint64_t quad_blocks = 0, thread_blocks = 0;
+    for (uint32_t r = 0; r < count; ++r) {
+        const uint64_t terms = (uint64_t)(offs[r + 1] - offs[r]) * W;
+        quad_blocks += (terms + SD_TERMS - 1) / SD_TERMS;
+        thread_blocks += (terms + SD_THREADS - 1) / SD_THREADS;
+    }
+    const bool quads = quad_blocks <= 2 * (uint64_t)sm_count() || quad_blocks < 2 * thread_blocks;
+    const uint32_t block_terms = quads ? SD_TERMS : SD_THREADS;
     std::vector<SdJob> jobs;
     std::vector<uint32_t> req_blocks(count + 1, 0);
     bool empty = false;
     for (uint32_t r = 0; r < count; ++r) {
         const uint32_t first = offs[r] * W, terms = (offs[r + 1] - offs[r]) * W;
-        for (uint32_t t = 0; t < terms; t += SD_TERMS)
-            jobs.push_back(SdJob{r, first + t, std::min<uint32_t>(SD_TERMS, terms - t), 0});
+        for (uint32_t t = 0; t < terms; t += block_terms)
+            jobs.push_back(SdJob{r, first + t, std::min<uint32_t>(block_terms, terms - t), 0});
         req_blocks[r + 1] = (uint32_t)jobs.size();
         empty |= terms == 0;
     }
@@ -1511,7 +1598,7 @@ void msm_sparse_direct(MsmWorkspace& ws, const MsmPrecomp<Fq>& pre, uint64_t nba
     uint32_t* h_words = reinterpret_cast<uint32_t*>(h_out + (size_t)count * XB);
     memset(h_words, 0xff, (size_t)count * 8);
     DV_CUDA(cudaMemcpyAsync(d_desc, h_desc, jb + rb + cb + 8, cudaMemcpyHostToDevice, st));
-    k_sparse_direct<<<(unsigned)jobs.size(), SD_THREADS, 0, st>>>(
+    (quads ? k_sparse_quads : k_sparse_threads)<<<(unsigned)jobs.size(), SD_THREADS, 0, st>>>(
         pre.table, nbases, pre.c, (int)W, d_idx, d_vals, reinterpret_cast<const SdJob*>(d_desc),
         reinterpret_cast<const uint32_t*>(d_desc + jb), d_partial, d_done, reinterpret_cast<XYZZ<Fq>*>(h_out),
         d_done + count, h_words);

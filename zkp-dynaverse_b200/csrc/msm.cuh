@@ -27,6 +27,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 
 #include "curve.cuh"
@@ -92,8 +93,8 @@ struct MsmPrecomp {
 // count canonical affine points (2 * sizeof(F) bytes each, all-zero for
 // infinity).  Throws InvalidArgument for non-canonical scalars.
 // Sparse MSMs over a resident table of window multiples, summed directly:
-// each (entry, window) term d T is formed by four lanes (double-and-add on
-// the signed c-bit digit d), then block and request sums.  For small
+// each (entry, window) term d T is formed by four lanes or one (double-and-add
+// on the signed c-bit digit d), then block and request sums.  For small
 // supports, where the bucket pipeline's launch chain dominates.  d_idx:
 // entry base indices (checked < nbases), d_vals: canonical scalars (checked),
 // offs (host, count + 1): entries of each request.  host_out: count
@@ -101,10 +102,24 @@ struct MsmPrecomp {
 void msm_sparse_direct(MsmWorkspace& ws, const MsmPrecomp<Fq>& pre, uint64_t nbases, const uint64_t* d_idx,
                        const uint32_t* d_vals, const uint32_t* offs, uint32_t count, uint8_t* host_out,
                        cudaStream_t stream);
-// Terms (entries x windows) up to which sparse calls take the direct path:
-// with a c = 8 table (32 windows) the direct path takes 143 and the bucket
-// pipeline 235 us for 256 entries, 202 and 219 for 512, 335 and 227 for 1024.
-constexpr uint64_t SPARSE_DIRECT_MAX_TERMS = 1u << 14;
+// Whether a sparse call of `count` requests with `terms` (entries x windows) in
+// all takes the direct path rather than the bucket pipeline: always up to
+// 16384 terms (c = 8, one request: 143 against 235 us for 256 entries, 202 and 219
+// for 512), never above 65536, and in between by what each has to pay.  The
+// pipeline carries a bucket set a request, which the device reduces and the host
+// normalises: 7 us + 1 us per 500 buckets.  The direct path pays (c + 1) / 2 us
+// per 1024 terms, and no less than one wave's 32768; its launch is 130 us the
+// shorter.  Whole calls of 32768 terms, direct and buckets: c = 8, 1 request 227
+// and 206 us, 2 220 and 232, 64 212 and 636; c = 10, 6 requests 243 and 240, 8
+// 237 and 256; c = 13, 4 279 and 269, 8 276 and 349; c = 16, 1 333 and 322, 2 326
+// and 354, 64 316 and 1967.  65536 terms: c = 8, 16 requests 353 and 311, 24 355
+// and 366; c = 16, 4 563 and 414, 6 562 and 565.
+inline bool msm_sparse_direct_pays(uint64_t terms, uint32_t count, int c) {
+    if (terms <= (1u << 14) || terms > (1u << 16)) return terms <= (1u << 14);
+    const double buckets = (double)(1u << (c - 1));
+    const double direct = (double)std::max<uint64_t>(terms, 1u << 15) / 1024 * (c + 1) / 2 - 130;
+    return count * (7 + buckets / 500) > direct;
+}
 
 // *d_points_bad, the error word of the points' conversion in the same stream,
 // is read before the wait and left in *points_bad.
