@@ -54,6 +54,27 @@ def test_ntt_batch_uneven_sizes_match_oracle(backend, oracle):
     assert backend.ntt_batch(parts[11], [16], [1]) == oracle.ntt(parts[11], "inverse")
 
 
+def test_ntt_batch_result_is_as_long_as_its_input_and_zero_past_the_transforms(backend, oracle):
+    """Input bytes past the transforms' give zero bytes, of a batch and of a
+    plan, whatever the memory of the returned object held before."""
+    parts = [oracle.uniform_fr(9200 + i, 4) for i in range(2)]
+    expect = b"".join(oracle.ntt(p, "forward") for p in parts)
+    values = b"".join(parts) + b"\x77" * 160
+    h = backend.register_bases(oracle.fixed_base_g1(oracle.uniform_fr(9210, 1)))
+    plan, _ = backend.batch_plan_create(h, [1], [2, 2])
+    try:
+        for call in (lambda: backend.ntt_batch(values, [2, 2]),
+                     lambda: backend.batch_plan_run(plan, oracle.uniform_fr(9211, 1), values, 1)[1]):
+            for _ in range(8):
+                junk = [bytes([i % 250 + 1]) * len(values) for i in range(500)]
+                del junk
+                assert call() == expect + bytes(160)
+        assert backend.ntt_batch(b"\x77" * 64, []) == bytes(64)
+    finally:
+        backend.batch_plan_destroy(plan)
+        backend.release_bases(h)
+
+
 def test_ntt_batch_device_matches_per_call(backend, oracle):
     import torch
     logs = [20, 10, 15, 18, 12, 19, 11, 16]

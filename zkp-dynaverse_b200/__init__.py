@@ -333,12 +333,18 @@ _bytes_of_size.restype = ctypes.py_object
 _bytes_of_size.argtypes = [ctypes.c_void_p, ctypes.c_ssize_t]
 
 
-def _result(n: int) -> bytes:
-    """A new, unfilled bytes object of n bytes for one library call to write
-    its result into before it is handed on (a new bytes object may be filled
-    until then).  A ctypes buffer would be cleared first, then copied by .raw and
+def _result(n: int, written: int | None = None) -> bytes:
+    """A new bytes object of n bytes for one library call to write its result
+    into before it is handed on (a new bytes object may be filled until then):
+    unfilled up to `written`, the length that the call writes (all of it where
+    not given), zeros from there on.  A ctypes buffer would be cleared first, then copied by .raw and
     once more by a slice: most of the time of calls with megabytes of results."""
-    return _bytes_of_size(None, n) if n > 0 else b""
+    if n <= 0:
+        return b""
+    out = _bytes_of_size(None, n)
+    if written is not None and written < n:
+        ctypes.memset(ctypes.cast(out, ctypes.c_void_p).value + written, 0, n - written)
+    return out
 
 
 def encode_fr(v: int) -> bytes:
@@ -1113,7 +1119,7 @@ class DvgpuBackend:
         forward)."""
         logs = np.ascontiguousarray(np.asarray(log_sizes, dtype=np.uint32))
         kd = None if kinds is None else np.ascontiguousarray(np.asarray(kinds, dtype=np.int32))
-        out = _result(max(1, len(values)))
+        out = _result(max(1, len(values)), FR_BYTES * sum(1 << int(x) for x in logs if x < 64))
         self._call("dvgpu_bn254_ntt_batch", _ptr(values), logs.ctypes.data if logs.size else None,
                    None if kd is None else kd.ctypes.data, len(logs), out)
         return out if len(values) else b""
@@ -1154,7 +1160,7 @@ class DvgpuBackend:
         results, concatenated NTT outputs)."""
         msm_out = ctypes.create_string_buffer(max(1, msm_count) * G1_BYTES)
         nbytes = 0 if ntt_values is None else len(ntt_values)
-        ntt_out = _result(max(1, nbytes))
+        ntt_out = _result(max(1, nbytes), self.batch_plan_buffers(plan).ntt_bytes)
         self._call("dvgpu_batch_plan_run", plan, _ptr(scalars), _ptr(ntt_values), msm_out, ntt_out)
         raw = msm_out.raw
         return [raw[i * G1_BYTES:(i + 1) * G1_BYTES] for i in range(msm_count)], (ntt_out if nbytes else b"")
