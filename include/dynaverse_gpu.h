@@ -686,7 +686,8 @@ int dvgpu_dynaverse_params_info(void* engine, uint64_t params, DvgpuDynaversePar
  * verified, written to proof. */
 int dvgpu_dynaverse_session_open(void* engine, uint64_t params, const uint8_t* public_inputs, const uint8_t* witness,
                                  uint64_t* session, uint8_t* proof, char* error, size_t error_capacity);
-/* -1 while a request of the session is unfinished (queued or being proved). */
+/* -1 while a request of the session is queued or its batch is being put on the
+ * GPU; once the GPU has the batch in full the call waits for it and closes. */
 int dvgpu_dynaverse_session_close(void* engine, uint64_t session, char* error, size_t error_capacity);
 /* The session's current witness (6n), instance (n), proof and anchor
  * distance (UpdateSession::current_witness / current_instance / proof /

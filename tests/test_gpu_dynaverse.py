@@ -282,6 +282,43 @@ def test_admission_budget_and_lifecycle_rules(dv):
         assert e.stats().resident_bytes == 0
 
 
+def test_close_waits_for_the_batch_that_the_gpu_has(dv):
+    """A close is refused until the session's batch is on the GPU in full, then
+    waits for it: it is accepted before the proof is done, the proof is the
+    oracle's, and the session is gone.  A second request of the session, queued
+    behind the batch, still refuses it."""
+    import time
+    n = 16
+    tx, ty = D.sample_trapdoors(15305, n)
+    pub, w = D.valid_instance(n)
+    with dv.DynaverseEngine(1 << 30, 8) as e:
+        ph = e.params_create(n, tx, ty)
+        for queued_behind in (False, True):
+            ref = D.Session(D.Params(n, tx, ty, "scalar"), pub, w)
+            s, _ = e.open_session(ph, pub, w)
+            first, second = _mul_edit(n, w, 3, 777), _mul_edit(n, w, 5, 778)
+            expect = [ref.update(*u).to_bytes() for u in (first, second)[:1 + queued_behind]]
+            tickets = [e.submit(s, *first)]
+            if queued_behind:
+                tickets.append(e.submit(s, *second))
+            while True:
+                called = time.monotonic_ns()
+                try:
+                    e.close_session(s)
+                    break
+                except dv.DvgpuError as err:
+                    assert err.status == -1 and "pending" in err.message
+            got = [e.wait(t) for t in tickets]
+            assert [g for g, _ in got] == expect
+            assert called + 200_000 < got[-1][1].done_ns  # the GPU's part takes a millisecond
+            if queued_behind:
+                assert called > got[0][1].done_ns
+            with pytest.raises(dv.DvgpuError) as err:
+                e.submit(s, *first)
+            assert "unknown session" in err.value.message
+        assert e.stats().sessions == 0
+
+
 @pytest.mark.parametrize("workload", ["hotspot", "spreading"])
 def test_reference_benchmark_workloads_n256(engine, workload):
     """The reference's own CPU benchmark sequences (crates/bench/src/bin/

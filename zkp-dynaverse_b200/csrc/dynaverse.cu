@@ -68,7 +68,6 @@
 #include <set>
 #include <string>
 #include <thread>
-#include <unordered_map>
 #include <unordered_set>
 #include <vector>
 
@@ -1360,13 +1359,16 @@ public:
         run([&] { id = open_impl(pid, pub, witness, proof); });
         return id;
     }
-    // Refused while any request of the session is unfinished when the call is
-    // made, queued or in a running batch: which of the two it is depends on
-    // how soon the worker looks at its queue.
+    // Refused while a request of the session is queued or its batch is being put
+    // on the GPU, both decided when the call is made: which of the two it is
+    // depends on how soon the worker looks at its queue.  A batch that the GPU has
+    // in full is waited for.
     void close_session(uint64_t id) {
         {
             std::lock_guard<std::mutex> lk(mu_);
-            if (unfinished_.count(id)) throw InvalidArgument("session has pending requests");
+            if (starting_.count(id) ||
+                std::any_of(queue_.begin(), queue_.end(), [&](const Request& r) { return r.session == id; }))
+                throw InvalidArgument("session has pending requests");
         }
         run([&] {
             std::lock_guard<std::mutex> lk(mu_);
@@ -1413,7 +1415,6 @@ public:
         if (!sessions_.count(session)) throw InvalidArgument("unknown session");
         r.ticket = next_ticket_++;
         outcomes_[r.ticket];
-        ++unfinished_[session];
         queue_.push_back(std::move(r));
         cv_.notify_all();
         return queue_.back().ticket;
@@ -1495,13 +1496,11 @@ private:
             }
             // the batch: FIFO, at most one request per session
             std::vector<Request> batch;
-            std::unordered_set<uint64_t> used;
             for (auto it = queue_.begin(); it != queue_.end() && batch.size() < max_batch_;) {
-                if (used.count(it->session)) {
+                if (!starting_.insert(it->session).second) {
                     ++it;
                     continue;
                 }
-                used.insert(it->session);
                 batch.push_back(std::move(*it));
                 it = queue_.erase(it);
             }
@@ -1528,9 +1527,8 @@ private:
                 o.res.batch_requests = (uint32_t)batch.size();
                 o.res.batch_id = (uint32_t)stat_batches_;
                 o.ready = true;
-                const auto u = unfinished_.find(batch[r].session);
-                if (--u->second == 0) unfinished_.erase(u);
             }
+            starting_.clear();
             stat_requests_ += batch.size();
             stat_batches_++;
             stat_largest_ = std::max<uint64_t>(stat_largest_, batch.size());
@@ -1603,7 +1601,7 @@ private:
     std::map<uint64_t, std::unique_ptr<Params>> params_;
     std::map<uint64_t, std::unique_ptr<Session>> sessions_;
     std::map<uint64_t, Outcome> outcomes_;
-    std::unordered_map<uint64_t, uint32_t> unfinished_;  // requests without an outcome, per session
+    std::unordered_set<uint64_t> starting_;  // sessions of the batch that is not on the GPU in full yet
     uint64_t next_id_ = 1, next_ticket_ = 1;
     uint64_t stat_requests_ = 0, stat_batches_ = 0, stat_largest_ = 0, stat_busy_ns_ = 0, stat_sparse_ = 0,
              stat_rebuilds_ = 0, stat_launches_ = 0;
@@ -2578,6 +2576,10 @@ void Engine::run_sparse(Params& P, std::vector<Job*>& jobs) {
     DV_CUDA(cudaMemcpyAsync(hout + ob + 4ull * B + 16, verd, eqs, cudaMemcpyDeviceToHost, st));
     const uint64_t w0 = now_ns();
     stat_enqueue_ns_ += w0 - e0;
+    {
+        std::lock_guard<std::mutex> lk(mu_);
+        for (const Job* j : jobs) starting_.erase(j->S->id);
+    }
     DV_CUDA(cudaStreamSynchronize(st));
     stat_wait_ns_ += now_ns() - w0;
     if (md.terms) {
