@@ -425,6 +425,50 @@ def test_msm_of_nearly_empty_lists(backend, oracle, value):
         assert backend.msm(pts, bytes(sc)) == _collected_sum(oracle, bases, bytes(sc)), k
 
 
+def test_msm_with_little_device_memory_left(dv, backend):
+    """A long G1 MSM takes 1.4 GB for its pairwise levels where they are to be
+    had, runs without them where not, and gives them back to a call that finds
+    no other memory; the sums are the same bytes, and the owner stays healthy."""
+    import torch
+    n = 1 << 20
+    stream = torch.cuda.current_stream().cuda_stream
+    scalars, powers, points = (torch.empty(k * n, dtype=torch.uint8, device="cuda") for k in (32, 32, 64))
+    values = torch.empty(32 << 23, dtype=torch.uint8, device="cuda")
+    backend.random_fr_device(6501, n, scalars.data_ptr(), stream)
+    backend.random_fr_device(6502, 1 << 23, values.data_ptr(), stream)
+    backend.fr_powers_device(values.data_ptr(), n, powers.data_ptr(), stream)
+    backend.fixed_base_device(powers.data_ptr(), n, False, points.data_ptr(), stream)
+    torch.cuda.synchronize()
+
+    def leave(nbytes):
+        torch.cuda.synchronize()
+        torch.cuda.empty_cache()
+        return torch.empty(torch.cuda.mem_get_info()[0] - nbytes, dtype=torch.uint8, device="cuda")
+
+    def msm(b):
+        return b.msm_device(points.data_ptr(), scalars.data_ptr(), n, stream=stream)
+
+    expect = msm(backend)
+    with dv.DvgpuBackend() as b:
+        held = leave(900 << 20)
+        assert msm(b) == expect  # without levels
+        del held
+        torch.cuda.empty_cache()
+        before = torch.cuda.mem_get_info()[0]
+        assert msm(b) == expect  # with them
+        assert before - torch.cuda.mem_get_info()[0] > 1 << 30
+        out = torch.empty_like(values)
+        held = leave(200 << 20)
+        b.ntt_device(values.data_ptr(), 1 << 23, 0, out.data_ptr(), stream)  # 0.4 GB of its own
+        assert msm(b) == expect
+        del held
+        ref = torch.empty_like(values)
+        backend.ntt_device(values.data_ptr(), 1 << 23, 0, ref.data_ptr(), stream)
+        assert torch.equal(out, ref)
+    del out, ref, values, points, powers, scalars
+    torch.cuda.empty_cache()
+
+
 @pytest.mark.parametrize("c", [8, 13])
 def test_sparse_direct_block_edges(backend, oracle, c):
     """One request around a block's 64 terms and around the direct path's

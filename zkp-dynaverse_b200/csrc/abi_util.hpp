@@ -29,6 +29,7 @@ int guarded(void* opaque, char* error, size_t cap, Fn&& fn) {
     if (b->retired) return fail(-4, "backend retired after an error; create a new backend", error, cap);
     try {
         DV_CUDA(cudaSetDevice(b->device));
+        const SpareRooms spare(b->msm.pairs);
         fn(*b);
         return 0;
     } catch (const InvalidArgument& e) {

@@ -1480,6 +1480,7 @@ private:
 
     void loop() {
         cudaSetDevice(device_);
+        const SpareRooms spare(ws1_.pairs, &ws2_.pairs, &ws3_.pairs);
         for (;;) {
             std::unique_lock<std::mutex> lk(mu_);
             cv_.wait(lk, [&] { return stop_ || !cmds_.empty() || !queue_.empty(); });

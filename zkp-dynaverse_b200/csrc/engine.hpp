@@ -63,14 +63,25 @@ struct DevBuf {
     size_t cap = 0;
     void* get(size_t bytes) {
         if (bytes <= cap && ptr) return ptr;
-        const uint64_t t0 = steady_ns();
         const size_t regrow = cap ? cap + cap / 2 : 0;
         release();
         size_t want = bytes < 256 ? 256 : bytes;
         if (regrow > want) want = regrow;
-        DV_CUDA(cudaMalloc(&ptr, want));
-        allocated(t0, want, false);
-        cap = want;
+        cudaError_t s = allocate(want);
+        if (s == cudaErrorMemoryAllocation && give_back_spare_rooms()) s = allocate(want);
+        cuda_check(s, "cudaMalloc");
+        return ptr;
+    }
+    // As get, but with headroom only up to `most` bytes, and null where the
+    // device has not that much memory left.
+    void* try_get(size_t bytes, size_t most) {
+        if (bytes <= cap && ptr) return ptr;
+        const size_t regrow = cap + cap / 2 < most ? cap + cap / 2 : most;
+        release();
+        cudaError_t s = allocate(regrow > bytes ? regrow : bytes);
+        if (s == cudaErrorMemoryAllocation && regrow > bytes) s = allocate(bytes);
+        if (s == cudaErrorMemoryAllocation) return nullptr;
+        cuda_check(s, "cudaMalloc");
         return ptr;
     }
     template <class T>
@@ -90,7 +101,52 @@ struct DevBuf {
     DevBuf() = default;
     DevBuf(const DevBuf&) = delete;
     DevBuf& operator=(const DevBuf&) = delete;
+
+  private:
+    cudaError_t allocate(size_t bytes) {
+        const uint64_t t0 = steady_ns();
+        const cudaError_t s = cudaMalloc(&ptr, bytes);
+        if (s != cudaSuccess) {
+            ptr = nullptr;
+            cudaGetLastError();  // not for the next launch's check
+            return s;
+        }
+        allocated(t0, bytes, false);
+        cap = bytes;
+        return s;
+    }
+    static bool give_back_spare_rooms();
 };
+
+// Buffers that the owner at work on this thread can do without (they make its
+// calls faster, and a later call takes them anew): while an object of this type
+// lives, an allocation of the thread that finds no memory frees them and tries
+// once more, so that they never cost a call that would run without them.
+struct SpareRooms {
+    DevBuf* rooms[3];
+    SpareRooms* outer;
+    explicit SpareRooms(DevBuf& a, DevBuf* b = nullptr, DevBuf* c = nullptr) : rooms{&a, b, c}, outer(current()) {
+        current() = this;
+    }
+    ~SpareRooms() { current() = outer; }
+    SpareRooms(const SpareRooms&) = delete;
+    SpareRooms& operator=(const SpareRooms&) = delete;
+    static SpareRooms*& current() {
+        static thread_local SpareRooms* top = nullptr;
+        return top;
+    }
+};
+inline bool DevBuf::give_back_spare_rooms() {
+    bool any = false;
+    for (SpareRooms* s = SpareRooms::current(); s; s = s->outer)
+        for (DevBuf* d : s->rooms) {
+            if (!d || !d->ptr) continue;
+            if (!any) cudaDeviceSynchronize();  // launches that use them; an error shows in the next call's check
+            any = true;
+            d->release();
+        }
+    return any;
+}
 
 // Grow-only pinned host buffer, with the same 1.5x headroom (freeing pinned
 // memory synchronises the device, so a stream of slowly growing requests

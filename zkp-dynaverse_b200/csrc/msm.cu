@@ -1118,10 +1118,24 @@ MsmPlan msm_plan_batch(uint32_t count, uint32_t max_set, uint64_t total, int for
 // level k runs while the list that it makes leaves PAIR_MIN_ROWS slots a
 // lane and a bucket still holds about four points.  Long lists go in chunks
 // of up to PAIR_CHUNK slots, so that the levels' room (about 150 bytes a
-// slot) stays below 2 GB whatever the launch.
+// slot: 1.43 GB for 2^20 points) stays below PAIR_ROOM bytes a workspace whatever
+// the launch.  Where the device has no such room left, the list is accumulated
+// without levels, and the room is given back to any other allocation of its owner.
 // MSM of 2^20 points: 4.11 ms without levels, 3.67 with levels down to 24 slots
 // a lane, 3.71 with 8 or 12; 32 proofs of 65536 gates 34.9 and 33.5 ms.
 constexpr uint64_t PAIR_MIN_ROWS = 20, PAIR_CHUNK = 12u << 20;
+constexpr size_t PAIR_ROOM = 2100u << 20;
+
+// The levels' room, or null.  A launch that is captured takes what an earlier one
+// of its shapes left: nothing can be allocated then.
+inline uint8_t* pair_room(MsmWorkspace& ws, size_t bytes, cudaStream_t st) {
+    if (ws.pairs.cap < bytes) {
+        cudaStreamCaptureStatus capture;
+        DV_CUDA(cudaStreamIsCapturing(st, &capture));
+        if (capture != cudaStreamCaptureStatusNone) return nullptr;
+    }
+    return static_cast<uint8_t*>(ws.pairs.try_get(bytes, PAIR_ROOM));
+}
 
 template <class F>
 void accumulate(MsmWorkspace& ws, const Affine<F>* pts, const uint32_t* d_sorted, const uint32_t* d_offsets,
@@ -1164,11 +1178,19 @@ void accumulate(MsmWorkspace& ws, const Affine<F>* pts, const uint32_t* d_sorted
             if (slots < PAIR_MIN_ROWS * lanes) break;
             caps.slots[levels++] = (uint32_t)slots;
         }
+        AccumChunk* d_chunks = nullptr;
+        uint32_t* d_last = nullptr;
+        uint8_t* room = nullptr;
         if (levels && chunks <= 1024) {
-            const size_t c1 = caps.slots[0], c2 = levels > 1 ? caps.slots[1] : 0;
-            size_t room_bytes = c1 * (8 + 64 + 32) + c2 * 64 + 16 * (PAIR_LEVELS_MAX + 4);
+            d_chunks = ws.pair_chunks.as<AccumChunk>(chunks);
+            d_last = ws.pair_offsets.as<uint32_t>((size_t)NB + 1);
+            size_t room_bytes = (size_t)caps.slots[0] * (8 + 64 + 32) + 16 * (PAIR_LEVELS_MAX + 4);
+            if (levels > 1) room_bytes += 64 * (size_t)caps.slots[1];
             for (int k = 1; k < levels; ++k) room_bytes += 4 * (size_t)caps.slots[k];
-            uint8_t* room = ws.pairs.as<uint8_t>(room_bytes);
+            room = pair_room(ws, room_bytes, st);  // last: an allocation could give it back
+        }
+        if (room) {
+            const size_t c1 = caps.slots[0], c2 = levels > 1 ? caps.slots[1] : 0;
             PairDescs descs{};
             size_t at = 0;
             const auto take = [&](size_t bytes) {
@@ -1180,8 +1202,6 @@ void accumulate(MsmWorkspace& ws, const Affine<F>* pts, const uint32_t* d_sorted
             uint4* buf[2] = {reinterpret_cast<uint4*>(take(64 * c1)), reinterpret_cast<uint4*>(take(64 * c2))};
             descs.first = reinterpret_cast<uint2*>(take(8 * c1));
             for (int k = 1; k < levels; ++k) descs.next[k - 1] = reinterpret_cast<uint32_t*>(take(4 * (size_t)caps.slots[k]));
-            AccumChunk* d_chunks = ws.pair_chunks.as<AccumChunk>(chunks);
-            uint32_t* d_last = ws.pair_offsets.as<uint32_t>((size_t)NB + 1);
             k_pair_chunks<<<1, 1024, 0, st>>>(d_offsets, NB, (uint32_t)chunks, levels, caps, d_chunks);
             DV_LAUNCH();
             const uint32_t pgrid = (uint32_t)sm_count() * PAIR_BLOCKS;

@@ -287,6 +287,7 @@ private:
 
     void loop() {
         cudaSetDevice(device_);
+        const SpareRooms spare(ws_.pairs);
         for (;;) {
             std::unique_lock<std::mutex> lk(mu_);
             cv_.wait(lk, [&] { return stop_ || !cmds_.empty() || !queue_.empty(); });
