@@ -425,6 +425,30 @@ def test_msm_of_nearly_empty_lists(backend, oracle, value):
         assert backend.msm(pts, bytes(sc)) == _collected_sum(oracle, bases, bytes(sc)), k
 
 
+@pytest.mark.parametrize("n", [1700000, 3300000])
+@pytest.mark.parametrize("skewed", ["half", "all"])
+def test_msm_chunks_that_do_not_fit(backend, oracle, n, skewed):
+    """Lists of two and of three chunks of pairwise levels, with half or all of
+    the scalars equal and all their digits the same: the chunk of that digit's
+    bucket is far over its room and summed from the sorted list, the middle one
+    of three is empty, and with half of them the last one goes through the
+    levels, its buckets behind the others'.  Over 64 bases in turn."""
+    c, digit = 16, 1 << 14
+    srs, _ = oracle.srs_g1(6601, 64)
+    bases = [srs[64 * i:64 * i + 64] for i in range(64)]
+    one = sum(digit << (c * w) for w in range(15)).to_bytes(32, "little")
+    sc = np.frombuffer(one * n, dtype=np.uint8).reshape(n, 32).copy()
+    if skewed == "half":
+        sc[::2] = np.frombuffer(oracle.uniform_fr(6602, (n + 1) // 2), dtype=np.uint8).reshape(-1, 32)
+    sc = sc.tobytes()
+    h = backend.register_bases((srs * (n // 64 + 1))[:64 * n])
+    try:
+        assert backend.precompute_bases(h, c) == c
+        assert backend.msm_resident_host(h, sc) == _collected_sum(oracle, bases, sc)
+    finally:
+        backend.release_bases(h)
+
+
 def test_msm_with_little_device_memory_left(dv, backend):
     """A long G1 MSM takes 1.4 GB for its pairwise levels where they are to be
     had, runs without them where not, and gives them back to a call that finds
