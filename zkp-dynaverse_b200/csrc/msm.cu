@@ -1121,8 +1121,11 @@ MsmPlan msm_plan_batch(uint32_t count, uint32_t max_set, uint64_t total, int for
 // slot: 1.43 GB for 2^20 points) stays below PAIR_ROOM bytes a workspace whatever
 // the launch.  Where the device has no such room left, the list is accumulated
 // without levels, and the room is given back to any other allocation of its owner.
-// MSM of 2^20 points: 4.11 ms without levels, 3.67 with levels down to 24 slots
-// a lane, 3.71 with 8 or 12; 32 proofs of 65536 gates 34.9 and 33.5 ms.
+// MSM of 2^20 points: 4.11 ms without levels, 3.55 with; 32 proofs of 65536 gates
+// 34.9 and 33.5 ms.  The least slots a lane, over 18 lists of 200000 to 4 M points
+// and 16 over tables of c = 16 and 13: 18 to 22 are within 1 % of each other at
+// every size; 14 is up to 6 % slower (150000 points, c = 16), 28 and 36 gain up to
+// 4 % at 200000 points and lose 4 to 9 % over the c = 13 table.
 constexpr uint64_t PAIR_MIN_ROWS = 20, PAIR_CHUNK = 12u << 20;
 constexpr size_t PAIR_ROOM = 2100u << 20;
 
@@ -1168,15 +1171,16 @@ void accumulate(MsmWorkspace& ws, const Affine<F>* pts, const uint32_t* d_sorted
     if constexpr (sizeof(F) == sizeof(Fq)) {
         const uint64_t lanes = (uint64_t)sm_count() * PAIR_BLOCKS * 128;
         const uint64_t chunks = std::max<uint64_t>(1, ((entries + NB) / 2 + PAIR_CHUNK - 1) / PAIR_CHUNK);
-        // room of each level for a chunk of even digits, an eighth over
-        const uint64_t e = entries / chunks + entries / chunks / 8 + 1024, b = NB / chunks + NB / chunks / 8 + 1024;
+        // slots of each level for a chunk of even digits; its room is an eighth over
+        const uint64_t e = entries / chunks, b = NB / chunks;
         PairCaps caps{};
         int levels = 0;
-        uint64_t slots = e;
+        uint64_t slots = e, room_slots = e + e / 8 + 1024;
         for (uint64_t per_bucket = entries / NB; levels < PAIR_LEVELS_MAX && per_bucket >= 4; per_bucket /= 2) {
             slots = (slots + b) / 2;
             if (slots < PAIR_MIN_ROWS * lanes) break;
-            caps.slots[levels++] = (uint32_t)slots;
+            room_slots = (room_slots + b + b / 8 + 1024) / 2;
+            caps.slots[levels++] = (uint32_t)room_slots;
         }
         AccumChunk* d_chunks = nullptr;
         uint32_t* d_last = nullptr;
