@@ -237,8 +237,6 @@ DV_INL F warp_batch_inverse(const F& x) {
 // scalars) then cost no more than with a thread a point.
 template <class F>
 struct Quad {
-    F c;
-
     DV_INL static int role() { return (int)(threadIdx.x & 3); }
     DV_INL static F from(const F& a, int r) { return shfl_idx(a, (int)(threadIdx.x & 28) + r); }
     DV_INL static bool flag(bool b, int r) { return __shfl_sync(0xffffffffu, (int)b, (int)(threadIdx.x & 28) + r) != 0; }

@@ -763,9 +763,6 @@ struct Fq2 {
         Fq::make_positive(d);
         return {Fq::redc(d), c1};
     }
-    DV_INL static PairOf<Fq2> mul2(const Fq2& a, const Fq2& b, const Fq2& c, const Fq2& d) {
-        return {mul(a, b), mul(c, d)};
-    }
     // (c0 + c1 u)^2 = (c0+c1)(c0-c1) + 2 c0 c1 u
     __device__ __noinline__ static Fq2 sqr(Fq2 a) {
         const Fq m = Fq::mul_inl(Fq::add_raw(a.c0, a.c1), Fq::sub(a.c0, a.c1));

@@ -178,12 +178,6 @@ DV_INL Lane lane_setup() {
     __syncthreads();
     return g;
 }
-DV_INL Fq shfl_xor_fq(const Fq& a, int m) {
-    Fq r;
-#pragma unroll
-    for (int w = 0; w < 8; ++w) r.v[w] = __shfl_xor_sync(FULL, a.v[w], m);
-    return r;
-}
 DV_INL Fq dbl_raw(const Fq& a, int by = 1) {
     Fq r;
     r.v[0] = a.v[0] << by;
@@ -201,7 +195,7 @@ DV_INL Fq reduce_top(const Fq& low, uint32_t top) {
 }
 // This lane's component of xi b: 9 b0 - b1 and 9 b1 + b0.
 DV_INL Fq xi_part(const Fq& b, int c) {
-    const Fq other = shfl_xor_fq(b, 1);
+    const Fq other = shfl_xor(b, 1);
     const Fq q = c ? other : neg_raw(other);
     const Fq s = dbl_raw(b, 3);
     uint32_t top = b.v[7] >> 29;
@@ -348,7 +342,7 @@ __device__ __noinline__ Fq g_cyc_sqr(Fq f, Lane g) {
     put_b(g, f, xf);
     __syncwarp();
     const int m = g.k == 0 || g.k == 3 ? 0 : (g.k == 2 || g.k == 5 ? 1 : 2);
-    const bool real = !(g.k & 1) && g.k != 3;
+    const bool real = !(g.k & 1);
     const Fq* a = sm(g.at + SM_A + 2 * m);
     const Fq* a3 = sm(g.at + SM_A + 2 * (m + 3));
     const Fq* b = sm(g.at + SM_B + 6 * m);
@@ -388,7 +382,7 @@ DV_INL Fq g_frob(const Lane& g, const Fq& f, int e) {
     if (e == 2) return Fq::mul(f, frob2(g.k));
     Fq2 s = frob1(g.k);
     if (e == 3) s = Fq2::mul_fq(s, frob2(g.k));
-    const Fq o = shfl_xor_fq(f, 1);
+    const Fq o = shfl_xor(f, 1);
     // component 0: f0 s0 + f1 s1; component 1: f0 s1 - f1 s0
     return Fq::mul_sub(o, s.c1, f, g.c ? s.c0 : Fq::neg(s.c0));
 }
