@@ -171,3 +171,46 @@ def test_product_of_unreduced_operand(p):
     cases += [(rng.randrange(p), rng.randrange(4 * p)) for _ in range(1500)] + [(p - 1, rng.randrange(3 * p, 4 * p)) for _ in range(300)]
     for x, y in cases:
         assert f.mul(_limbs(x), _limbs(y)) == x * y * r_inv % p
+
+
+@pytest.mark.parametrize("p", [Q, R])
+def test_product_with_unreduced_rows(p):
+    """Fp::mul_lazy the other way round, a < 2p times b < p, as Fq2::sqr and the
+    scaling after a transform have it: below 2p, no carry lost."""
+    f, rng, r_inv = Field(p), random.Random(10), pow(1 << 256, -1, p)
+    edge_a = [0, 1, p - 1, p, p + 1, 2 * p - 2, 2 * p - 1]
+    cases = [(x, y) for x in edge_a for y in (0, 1, p - 1, p - 2, p - (p & M32), (1 << 253) - 1)]
+    cases += [(rng.randrange(2 * p), rng.randrange(p)) for _ in range(1500)]
+    cases += [(rng.randrange(2 * p - 99, 2 * p), rng.randrange(p - (1 << 200), p)) for _ in range(300)]
+    for x, y in cases:
+        assert f.mul(_limbs(x), _limbs(y)) == x * y * r_inv % p
+
+
+class RawField(Field):
+    def finish(self, e, o, high=0):
+        r = _value(e[1:]) + _value(o) + high
+        assert r < 1 << 256
+        return r
+
+
+@pytest.mark.parametrize("p", [Q, R])
+def test_reduction_of_large_sums(p):
+    """Fp::redc_raw: a high half of up to 4.27 p keeps the sum below 2^256, and
+    below the high half plus p and p / 2^32."""
+    f, rng, r_inv = RawField(p), random.Random(11), pow(1 << 256, -1, p)
+    top = 427 * p // 100
+    lows = [0, 1, M32, (1 << 256) - 1, (1 << 256) - (1 << 32), p << 2]
+    cases = [(h, low) for h in (0, 1, p, 2 * p, 4 * p, top - 1, top) for low in lows]
+    cases += [(rng.randrange(top + 1), rng.randrange(1 << 256)) for _ in range(1500)]
+    for h, low in cases:
+        t = h << 256 | low
+        got = f.redc(_limbs(t, 16))
+        assert got % p == t * r_inv % p and got <= h + p + (p >> 32)
+
+
+def test_quotient_estimate_from_the_top_bits():
+    """reduce_top of the pairing: for v < 10 q with top = v >> 252, 21 top / 64
+    is the quotient by q or one less, at both ends of every top's values."""
+    for top in range((10 * Q - 1 >> 252) + 1):
+        for v in (top << 252, min((top + 1 << 252) - 1, 10 * Q - 1)):
+            assert v // Q - 1 <= top * 21 >> 6 <= v // Q

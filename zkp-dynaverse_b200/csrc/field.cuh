@@ -12,9 +12,14 @@
 //    then always lands on an even-aligned register pair (one multiply-add
 //    instruction), also after the shift by one limb, which makes O the new
 //    E and E without two limbs the new O: no moves, no re-split additions.
+//    (Aligned and unaligned partial products in accumulators of their own:
+//    Emmart, Luitjens, Weems and Woolley, "Optimizing modular multiplication for
+//    NVIDIA's Maxwell GPUs", ARITH 2016, there for 16-bit halves.)
 //  - With N = (p (-p^-1 mod 2^32) + 1) / 2^32, T + t0 p (-p^-1 mod 2^32) is
 //    divisible by 2^32 and its quotient is (T >> 32) + t0 N (t0 the low limb):
-//    a reduction step needs no product for its multiplier.  N < p, but the
+//    a reduction step needs no product for its multiplier (Orup, "Simplifying
+//    quotient determination in high-radix modular multiplication", ARITH
+//    1995).  N < p, but the
 //    steps no longer keep T below 2p, so the last two take the multiplier
 //    m = -t0 / p mod 2^32 and p.  Bounds: T < 2^33 p < 2^288 before every
 //    step, below 2p after the last.
@@ -171,8 +176,9 @@ struct __align__(16) Fp {  // 16-byte aligned: global copies move as 128-bit acc
         reduce_once(r.v);
         return r;
     }
-    // The same without the last subtraction, for a < p and b < 4p (in this
-    // order: the rows are a's): below 1.76 p, with T below 2.94 p 2^32 < 2^288.
+    // The same without the last subtraction.  The rows are a's, so the order
+    // matters.  a < p and b < 4p: below 1.76 p, with T below 1.94 p 2^32.  a < 2p and
+    // b < p: below 1.38 p, with T below 2.94 p 2^32 < 2^288.
     DV_INL static Fp mul_lazy(const Fp& a, const Fp& b) {
         constexpr Words N = reduction_words();
         uint32_t e[8], o[8], t[8];
