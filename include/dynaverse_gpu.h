@@ -113,13 +113,14 @@ int dvgpu_bn254_fixed_base_g2_checked(void* owner, const uint8_t* scalars, size_
                                       size_t error_capacity);
 /* G2 check kernel diagnostics (native/include/dynaverse_g2_experiments.h:6-17,
  * bound by crates/gpu/src/g2_validation.rs:91-94).  config: threads 64, 128
- * or 256 is the check kernel's block size; schedule, layout and fused (0 or
+ * or 256 is the check kernels' block size; schedule, layout and fused (0 or
  * 1) name the reference's experimental variants and are accepted and kept
- * without effect (this library has one check kernel, with the fixed-base
- * normalisation always fused).  resources: the check kernel's attributes and
- * theoretical occupancy at the configured block size, and those of the
- * checked G2 fixed-base generation.  experiment stats: no repacking
- * (repack fields 0); subgroup_kernel_ns sums the check kernel's device time. */
+ * without effect (this library takes four lanes a point up to 32 points an SM
+ * and one beyond, with the fixed-base normalisation always fused).
+ * resources: attributes and theoretical occupancy at the configured block
+ * size of that one of the two check kernels that leaves fewer blocks on an SM,
+ * and those of the checked G2 fixed-base generation.  experiment stats: no repacking
+ * (repack fields 0); subgroup_kernel_ns sums the check kernels' device time. */
 typedef struct DvgpuG2KernelConfig {
     uint32_t threads, schedule, layout, fused;
 } DvgpuG2KernelConfig;

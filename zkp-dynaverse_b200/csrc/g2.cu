@@ -1,4 +1,6 @@
 // G2 validation and fixed-base generation kernels (see g2.cuh).
+#include <climits>
+
 #include "g2.cuh"
 
 namespace dv {
@@ -315,12 +317,22 @@ void g2_check_launch(const uint8_t* d_wire, uint64_t n, uint32_t algorithm, uint
 }
 
 void g2_kernel_resources(unsigned threads, DvgpuG2KernelResources& out) {
-    int dev = 0, max_threads = 0, blocks = 0, nblocks = 0;
+    int dev = 0, max_threads = 0, blocks = INT_MAX, nblocks = 0;
     DV_CUDA(cudaGetDevice(&dev));
     DV_CUDA(cudaDeviceGetAttribute(&max_threads, cudaDevAttrMaxThreadsPerMultiProcessor, dev));
     cudaFuncAttributes a{}, na{};
-    DV_CUDA(cudaFuncGetAttributes(&a, k_g2_check<3>));  // the default algorithm's kernel
-    DV_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k_g2_check<3>, (int)threads, 0));
+    // the default algorithm's kernels, a thread and a quad a point: of the two the
+    // one that leaves fewer blocks on an SM
+    for (auto kernel : {k_g2_check<3>, k_g2_check_quads<3>}) {
+        cudaFuncAttributes ka{};
+        int kb = 0;
+        DV_CUDA(cudaFuncGetAttributes(&ka, kernel));
+        DV_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&kb, kernel, (int)threads, 0));
+        if (kb < blocks || (kb == blocks && ka.numRegs > a.numRegs)) {
+            blocks = kb;
+            a = ka;
+        }
+    }
     // the checked fixed-base normalisation is fused into its generation kernel
     DV_CUDA(cudaFuncGetAttributes(&na, k_fb_generate<Fq2>));
     DV_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nblocks, k_fb_generate<Fq2>, 128, 0));
