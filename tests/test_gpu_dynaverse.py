@@ -99,6 +99,26 @@ def test_every_affected_size_and_the_empty_set(engine):
         engine.close_session(s)
 
 
+def test_vanishing_values_by_one_block_and_by_all(engine):
+    """Affected sets around the sizes where the vanishing polynomial's values
+    go from one block to the whole GPU, and around powers of two."""
+    n = 1024  # rebuild interval 32
+    ph, P = _setup(engine, n, 15403)
+    pub, w = D.valid_instance(n)
+    for count in (4, 5, 6, 7, 8, 15):
+        s, _ = engine.open_session(ph, pub, w)
+        ref = D.Session(P, pub, w, verify=False)
+        idx, v = [], []
+        for g, val in enumerate(D.ints(O.uniform_fr(15404 + count, count))):
+            ii, vv = _mul_edit(n, w, 61 * g + 2, val)
+            idx += ii
+            v += vv
+        expect = ref.update(idx, v, verify=False)
+        assert expect.delta is not None
+        assert engine.update(s, idx, v) == expect.to_bytes(), count
+        engine.close_session(s)
+
+
 def test_invalid_updates_are_rejected_without_state_change(engine, dv):
     n = 32
     ph, _ = _setup(engine, n, 15302)

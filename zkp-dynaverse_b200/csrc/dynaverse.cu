@@ -617,10 +617,12 @@ __global__ void k_dv_geom(FieldCtx c) {
 // product split over its lanes, then an inverse transform of size N in
 // shared memory.  The chain is about a / 32 + log N + 5 products, against a
 // for the product taken one factor at a time.  The N values are a N products,
-// too many for one SM once a is in the tens (a = 100: 128 us in this kernel,
-// 31 us for both): k_dv_vanish_values then spreads them over the GPU, a
+// soon too many for one SM (a = 100: 128 us in this kernel, 31 us for both):
+// k_dv_vanish_values then spreads them over the GPU, a
 // warp a value, into the job's matrix scratch (a a elements, unused yet).
-constexpr uint32_t VANISH_SPLIT = 16;  // affected points up to which one block does it all
+// With one block / with both, a lone job and 16 alike: a = 4 14 / 16 us, 6 19 / 17,
+// 8 to 24 27 / 18.
+constexpr uint32_t VANISH_SPLIT = 5;  // affected points up to which one block does it all
 DV_INL Fr vanish_value(const Fr& y, const Fr* x, uint32_t a, uint32_t lane) {
     Fr p = Fr::one();
     for (uint32_t k = lane; k < a; k += 32) p = Fr::mul(p, Fr::sub(y, x[k]));
