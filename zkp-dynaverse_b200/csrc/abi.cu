@@ -426,14 +426,14 @@ void sparse_run(Backend& b, const ResidentBases& rb, const uint64_t* d_idx, cons
                 const std::vector<uint32_t>& offs, uint8_t* out, cudaStream_t st) {
     const uint32_t count = (uint32_t)offs.size() - 1;
     const uint64_t k_total = offs[count];
-    uint32_t* bad = b.err.as<uint32_t>(1);
-    DV_CUDA(cudaMemsetAsync(bad, 0xff, sizeof(uint32_t), st));
     if (rb.pre_c && msm_sparse_direct_pays(k_total * (uint64_t)rb.pre_windows, count, rb.pre_c)) {
         const MsmPrecomp<Fq> pre{rb.pre_table.view<G1A>(), rb.pre_c, rb.pre_windows};
         msm_sparse_direct(b.msm, pre, rb.n, d_idx, reinterpret_cast<const uint32_t*>(d_vals), offs.data(), count,
                           out, st);
         return;
     }
+    uint32_t* bad = b.err.as<uint32_t>(1);
+    DV_CUDA(cudaMemsetAsync(bad, 0xff, sizeof(uint32_t), st));
     if (rb.pre_c) {
         G1A* gathered = b.conv_points.as<G1A>(k_total * rb.pre_windows);
         gather_table<Fq>(rb.pre_table.view<G1A>(), rb.n, rb.pre_windows, d_idx, k_total, gathered, bad, st);
