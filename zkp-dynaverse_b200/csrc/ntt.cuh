@@ -93,7 +93,7 @@ constexpr int BATCH_TILE_MIN = 8, BATCH_TILE_DEFAULT = 11, BATCH_TILE_MAX = 12;
 struct NttBatch {
     DevBuf descs, tiles, ctl, work, errs;
     uint32_t count = 0, ntiles = 0, grid = 0;
-    int radix_log = 2;  // register round of the kernel: radix 2, 4 or 8
+    int radix_log = 1;  // register round of the kernel: radix 2, 4 or 8
     int tile_log = BATCH_TILE_DEFAULT;
     uint64_t elements = 0;
     std::vector<uint64_t> work_off;
