@@ -1164,7 +1164,7 @@ void accumulate(MsmWorkspace& ws, const Affine<F>* pts, const uint32_t* d_sorted
                                                                chunk);
         DV_LAUNCH();
         // long chains are rare: a small grid loops over the queue
-        k_fixup_long<F><<<std::min<uint32_t>(T / FIX_SHORT + 1, (uint32_t)sm_count() * 2), 256, 0, st>>>(
+        k_fixup_long<F><<<std::min<uint32_t>(T / FIX_SHORT / 8 + 1, (uint32_t)sm_count() * 2), 256, 0, st>>>(
             d_pgid, d_ppt, T, d_buckets, d_fix_list, d_fix_count, chunk);
         DV_LAUNCH();
     };
