@@ -104,8 +104,8 @@ void msm_sparse_direct(MsmWorkspace& ws, const MsmPrecomp<Fq>& pre, uint64_t nba
                        cudaStream_t stream);
 // Whether a sparse call of `count` requests with `terms` (entries x windows) in
 // all takes the direct path rather than the bucket pipeline: always up to
-// 16384 terms (c = 8, one request: 143 against 235 us for 256 entries, 202 and 219
-// for 512), never above 65536, and in between by what each has to pay.  The
+// 16384 terms (c = 8, one request: 119 us for 256 entries, 200 for 512, where the
+// pipeline's 195 begin), never above 65536, and in between by what each has to pay.  The
 // pipeline carries a bucket set a request, which the device reduces and the host
 // normalises: 7 us + 1 us per 500 buckets.  The direct path pays (c + 1) / 2 us
 // per 1024 terms, and no less than one wave's 32768; its launch is 130 us the
