@@ -322,7 +322,9 @@ typedef struct DvgpuMsmPhaseTimes {
 int dvgpu_msm_timeline(void* backend, int enable, DvgpuMsmPhaseTimes* out);
 
 /* Seeded synthetic inputs on the device: n uniform Fr scalars (canonical),
- * and the powers tau^0..tau^(n-1) of a canonical device scalar. */
+ * and the powers tau^0..tau^(n-1) of a canonical device scalar.  These and the
+ * twist points below are enqueued on `stream`; with NULL (the owner's stream)
+ * the call returns once the output is there. */
 int dvgpu_random_fr_device(void* backend, uint64_t seed, size_t n, uint8_t* d_out, void* stream, char* error,
                            size_t error_capacity);
 int dvgpu_fr_powers_device(void* backend, const uint8_t* d_tau, size_t n, uint8_t* d_out, void* stream, char* error,

@@ -231,3 +231,21 @@ def test_ntt_reports_the_first_bad_value_and_recovers(backend, oracle, logn):
         with pytest.raises(Exception, match=rf"index {first}\b"):
             on_device(bytes(bad))
         assert on_device(good) == expect
+
+
+def test_generators_on_the_owners_stream_return_with_their_output(backend):
+    """The last bytes, which the kernel writes last, read at once on another
+    stream."""
+    import torch
+    n = 1 << 25
+    tau = torch.zeros(32, dtype=torch.uint8, device="cuda")
+    tau[0] = 3
+    calls = [lambda p: backend.random_fr_device(77, n, p), lambda p: backend.fr_powers_device(tau.data_ptr(), n, p),
+             lambda p: backend.random_twist_device(78, n // 128, p)]
+    for call, size in zip(calls, (32 * n, 32 * n, n)):
+        out = torch.zeros(size, dtype=torch.uint8, device="cuda")
+        torch.cuda.synchronize()
+        call(out.data_ptr())
+        last = out[-32:].cpu()
+        torch.cuda.synchronize()
+        assert last.any() and torch.equal(last, out[-32:].cpu())

@@ -1138,11 +1138,20 @@ extern "C" int dvgpu_msm_timeline(void* opaque, int enable, DvgpuMsmPhaseTimes* 
     }
 }
 
+namespace {
+// On the owner's stream, which no caller can order its own work behind, the
+// generators return with their output in place.
+void generated(Backend& b, void* stream) {
+    if (!stream) DV_CUDA(cudaStreamSynchronize(b.stream));
+}
+}  // namespace
+
 extern "C" int dvgpu_random_fr_device(void* opaque, uint64_t seed, size_t n, uint8_t* d_out, void* stream,
                                       char* error, size_t cap) {
     return guarded(opaque, error, cap, [&](Backend& b) {
         require(!n || d_out, "null output");
         dv::random_fr_launch(seed, n, d_out, pick(b, stream));
+        generated(b, stream);
     });
 }
 
@@ -1151,6 +1160,7 @@ extern "C" int dvgpu_g2_random_twist_device(void* opaque, uint64_t seed, size_t 
     return guarded(opaque, error, cap, [&](Backend& b) {
         require(!n || d_out, "null output");
         dv::random_twist_launch(seed, n, d_out, pick(b, stream));
+        generated(b, stream);
     });
 }
 
@@ -1159,6 +1169,7 @@ extern "C" int dvgpu_fr_powers_device(void* opaque, const uint8_t* d_tau, size_t
     return guarded(opaque, error, cap, [&](Backend& b) {
         require(d_tau && (!n || d_out), "null buffers");
         dv::powers_launch(d_tau, n, d_out, pick(b, stream));
+        generated(b, stream);
     });
 }
 
