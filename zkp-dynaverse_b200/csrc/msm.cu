@@ -1121,12 +1121,14 @@ MsmPlan msm_plan_batch(uint32_t count, uint32_t max_set, uint64_t total, int for
 // slot: 1.43 GB for 2^20 points) stays below PAIR_ROOM bytes a workspace whatever
 // the launch.  Where the device has no such room left, the list is accumulated
 // without levels, and the room is given back to any other allocation of its owner.
-// MSM of 2^20 points: 4.11 ms without levels, 3.55 with; 32 proofs of 65536 gates
+// MSM of 2^20 points: 4.11 ms without levels, 3.57 with; 32 proofs of 65536 gates
 // 34.9 and 33.5 ms.  The least slots a lane, over 18 lists of 200000 to 4 M points
-// and 16 over tables of c = 16 and 13: 18 to 22 are within 1 % of each other at
+// and 16 over tables of c = 16 and 13: 18 to 22 are within 1.5 % of each other at
 // every size; 14 is up to 6 % slower (150000 points, c = 16), 28 and 36 gain up to
-// 4 % at 200000 points and lose 4 to 9 % over the c = 13 table.
-constexpr uint64_t PAIR_MIN_ROWS = 20, PAIR_CHUNK = 12u << 20;
+// 4 % at 200000 points and lose 4 to 9 % over the c = 13 table.  18, because lists
+// with few full buckets gain by every level (300001 scalars 0 and 1: 1.06 ms, with
+// 20 1.90).
+constexpr uint64_t PAIR_MIN_ROWS = 18, PAIR_CHUNK = 12u << 20;
 constexpr size_t PAIR_ROOM = 2100u << 20;
 
 // The levels' room, or null.  A launch that is captured takes what an earlier one
